@@ -593,22 +593,66 @@ template int launch_validate<int32_t>(cudaStream_t, int64_t, int64_t, int64_t, c
 template int launch_validate<int64_t>(cudaStream_t, int64_t, int64_t, int64_t, const int64_t *,
                                       const int64_t *, int, int *);
 
-// Row pointers of a row-sorted COO: entry i's predecessor and its own row bound the
-// pointer entries it writes (each written once); a decrease or a row outside [0, m)
-// clears *sorted instead.
+// Row pointers of a COO whose row indices are non-decreasing, in two steps, because a COO in
+// random order must not pay for the pointers of an order that it does not have: writing an entry's
+// pointers before the order was known took 12 s for 16M entries over 10^6 rows in random order
+// (every increase wrote the whole gap, a thread alone); the check now ends that call within its
+// first loads.
+
+// Clears *sorted where a row index decreases or lies outside [base, base + m).  Bound by the read
+// of the indices; a warp leaves once any warp has found a violation.
+template <typename I>
+__global__ void coo_sorted_kernel(int64_t nnz, const I *__restrict__ rowind, int base, int64_t m,
+                                  volatile int *sorted) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < nnz; i0 += stride) {
+        if (!*sorted) return;
+        const int64_t i = i0 + threadIdx.x;
+        if (i >= nnz) return;
+        const int64_t cur = (int64_t)rowind[i] - base;
+        const int64_t prev = i == 0 ? 0 : (int64_t)rowind[i - 1] - base;
+        if (cur < prev || cur < 0 || cur >= m) *sorted = 0;
+    }
+}
+
+// Entry i writes the pointers of the rows after its predecessor's up to its own (entry nnz, past
+// the end, those of the last rows).  Gaps of more than 32 rows are written by the whole warp.
 template <typename I>
 __global__ void coo_rowptr_kernel(int64_t nnz, const I *__restrict__ rowind, int base, int64_t m,
-                                  I *__restrict__ ptr_out, int *sorted) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= nnz;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t prev = i == 0 ? -1 : (int64_t)rowind[i - 1] - base;
-        const int64_t cur = i == nnz ? m : (int64_t)rowind[i] - base;
-        if (cur < prev || cur > m || (i < nnz && cur == m) || prev >= m) {
-            atomicExch(sorted, 0);
-            continue;
+                                  I *__restrict__ ptr_out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 <= nnz; i0 += stride) {
+        const int64_t i = i0 + lane;
+        int64_t prev = 0, cur = -1;  // rows prev + 1 .. cur: none
+        if (i <= nnz) {
+            prev = i == 0 ? -1 : (int64_t)rowind[i - 1] - base;
+            cur = i == nnz ? m : (int64_t)rowind[i] - base;
         }
-        for (int64_t r = prev + 1; r <= cur; ++r) ptr_out[r] = (I)(i + base);
+        const bool wide = cur - prev > 32;
+        if (!wide)
+            for (int64_t r = prev + 1; r <= cur; ++r) ptr_out[r] = (I)(i + base);
+        for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1) {
+            const int l = __ffs(todo) - 1;
+            const int64_t p = __shfl_sync(0xffffffffu, prev, l), c = __shfl_sync(0xffffffffu, cur, l);
+            for (int64_t r = p + 1 + lane; r <= c; r += 32) ptr_out[r] = (I)(i0 + l + base);
+        }
     }
+}
+
+template <typename I>
+static int coo_row_pointers_i(cudaStream_t s, int64_t m, int64_t nnz, const I *rowind, int base, I *ptr_out,
+                              int *flag, int *sorted_host) {
+    int64_t blocks = ceil_div(nnz + 1, 256);
+    if (blocks > 152 * 64) blocks = 152 * 64;
+    if (nnz > 0) coo_sorted_kernel<I><<<(unsigned)blocks, 256, 0, s>>>(nnz, rowind, base, m, flag);
+    int rc = check_cuda(cudaGetLastError(), "coo_sorted_kernel");
+    if (!rc) rc = check_cuda(cudaMemcpyAsync(sorted_host, flag, sizeof(int), cudaMemcpyDeviceToHost, s),
+                             "coo plan: flag");
+    if (!rc) rc = check_cuda(cudaStreamSynchronize(s), "coo plan: sync");
+    if (rc || !*sorted_host) return rc;
+    coo_rowptr_kernel<I><<<(unsigned)blocks, 256, 0, s>>>(nnz, rowind, base, m, ptr_out);
+    return check_cuda(cudaGetLastError(), "coo_rowptr_kernel");
 }
 
 int coo_row_pointers(cudaStream_t s, int itype, int64_t m, int64_t nnz, const void *rowind, int base,
@@ -616,22 +660,15 @@ int coo_row_pointers(cudaStream_t s, int itype, int64_t m, int64_t nnz, const vo
     int *flag = nullptr;
     int rc = check_cuda(cudaMallocAsync((void **)&flag, sizeof(int), s), "coo plan: flag");
     if (rc) return rc;
-    const int one = 1;
-    rc = check_cuda(cudaMemcpyAsync(flag, &one, sizeof(int), cudaMemcpyHostToDevice, s), "coo plan: flag");
+    rc = check_cuda(cudaMemsetAsync(flag, 1, sizeof(int), s), "coo plan: flag");  // any value but 0
     if (!rc) {
-        int64_t blocks = ceil_div(nnz + 1, 256);
-        if (blocks > 152 * 64) blocks = 152 * 64;
         if (itype == GSA_IDX32)
-            coo_rowptr_kernel<int32_t><<<(unsigned)blocks, 256, 0, s>>>(nnz, (const int32_t *)rowind, base, m,
-                                                                         (int32_t *)ptr_out, flag);
+            rc = coo_row_pointers_i<int32_t>(s, m, nnz, (const int32_t *)rowind, base, (int32_t *)ptr_out, flag,
+                                             sorted_host);
         else
-            coo_rowptr_kernel<int64_t><<<(unsigned)blocks, 256, 0, s>>>(nnz, (const int64_t *)rowind, base, m,
-                                                                         (int64_t *)ptr_out, flag);
-        rc = check_cuda(cudaGetLastError(), "coo_rowptr_kernel");
+            rc = coo_row_pointers_i<int64_t>(s, m, nnz, (const int64_t *)rowind, base, (int64_t *)ptr_out, flag,
+                                             sorted_host);
     }
-    if (!rc) rc = check_cuda(cudaMemcpyAsync(sorted_host, flag, sizeof(int), cudaMemcpyDeviceToHost, s),
-                             "coo plan: flag");
-    if (!rc) rc = check_cuda(cudaStreamSynchronize(s), "coo plan: sync");
     cudaFreeAsync(flag, s);
     return rc;
 }
