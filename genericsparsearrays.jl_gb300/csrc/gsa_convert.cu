@@ -658,7 +658,7 @@ static int coo_row_pointers_i(cudaStream_t s, int64_t m, int64_t nnz, const I *r
 int coo_row_pointers(cudaStream_t s, int itype, int64_t m, int64_t nnz, const void *rowind, int base,
                      void *ptr_out, int *sorted_host) {
     int *flag = nullptr;
-    int rc = check_cuda(cudaMallocAsync((void **)&flag, sizeof(int), s), "coo plan: flag");
+    int rc = check_cuda(scratch_alloc((void **)&flag, sizeof(int), s), "coo plan: flag");
     if (rc) return rc;
     rc = check_cuda(cudaMemsetAsync(flag, 1, sizeof(int), s), "coo plan: flag");  // any value but 0
     if (!rc) {

@@ -48,6 +48,7 @@ struct gsa_plan {
     gsa_bin_order order{};                // its arrays (device pointers)
     const gsa_bin_order *bin_view = nullptr;  // device copy of `order`
     void *mem = nullptr;
+    int device = 0;                       // the device of mem and coo_ptr
     // COO plans (gsa_coo_plan_create): row pointers of a row-sorted COO (owned), the rest of
     // the plan describing them; coo_sorted = 0 leaves the COO kernel in charge
     int coo = 0, coo_sorted = 0;
@@ -351,6 +352,11 @@ void radix_sort_inputs(void *ws, int64_t n, uint64_t **keys, uint32_t **perm);
 int radix_sort_pairs(cudaStream_t s, void *ws, int64_t n, int total_bits, uint64_t **keys_out, uint32_t **perm_out);
 int radix_bits_for(int64_t count);  // bits that values 0 .. count - 1 need
 
+// Stream-ordered scratch from the library's own pool of the current device (gsa_capi.cu): given
+// back with cudaFreeAsync on a stream that is ordered after its last use, or with cudaFree once
+// the device has been synchronized (cudaFree waits for nothing on such memory).
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s);
+
 // Scratch of one call: the caller's buffer, or a stream-ordered allocation freed on the
 // same stream when the call returns.
 struct Workspace {
@@ -369,7 +375,7 @@ struct Workspace {
             bytes = user_bytes;
             return GSA_OK;
         }
-        cudaError_t e = cudaMallocAsync(&p, need, stream);
+        cudaError_t e = scratch_alloc(&p, need, stream);
         if (e != cudaSuccess) {
             cudaGetLastError();
             return fail(GSA_ERR_ALLOC, "stream-ordered workspace allocation of %zu bytes failed: %s",

@@ -23,9 +23,7 @@
 // Without a plan such a row is one group's work like any other.
 //
 // Every row's summation order is fixed, so results are deterministic.
-#include <algorithm>
 #include <atomic>
-#include <vector>
 
 #include "gsa_rows.cuh"
 
@@ -419,205 +417,6 @@ size_t rowblock_workspace_size(const Plan *plan, size_t vsize, int64_t k) {
     cv.take<int>((size_t)(nlong * k));
     cv.take<unsigned char>((size_t)(nchunks * k) * vsize + 16);
     return align_up(cv.off, 256);
-}
-
-// ---------------------------------------------------------------------------
-// Plans.
-
-// Bin of a row of len <= CHUNK entries and its lanes per row: rows of equal length up to
-// 32 (a lane each), then for 32 < len <= 512 the G = 2, 4, 8 or 16 lanes with 16 <
-// ceil(len / G) <= 32 and one bin per value of ceil(len / G): every lane of a warp does
-// the same number of multiply-adds, 17 to 32, before the width-G reduction.
-constexpr int NBINS = 97;
-constexpr int64_t BIN_SEGMENT = 32768;  // rows per segment of the bin order
-static int bin_of(int64_t len) {
-    if (len <= 32) return (int)len;
-    int lg = 1;
-    while (((int64_t)32 << lg) < len) ++lg;  // G = 2^lg lanes: 32 * G >= len
-    const int64_t q = (len + ((int64_t)1 << lg) - 1) >> lg;  // 17 .. 32
-    return 33 + (lg - 1) * 16 + (int)(q - 17);
-}
-static int bin_lanes(int b) { return b <= 32 ? 1 : 1 << (1 + (b - 33) / 16); }
-
-// Lane utilisation of the natural order: the fraction of lane-iterations that do a
-// multiply-add when a warp of 32 rows runs G lanes per row (G from the rows' average, as
-// warp_extent and dispatch_lanes pick it) and each pass lasts as long as its longest row.
-static double natural_utilisation(const std::vector<int64_t> &len, const std::vector<uint32_t> &mask) {
-    double busy = 0, held = 0;
-    const int64_t n = (int64_t)len.size();
-    for (int64_t w0 = 0; w0 < n; w0 += 32) {
-        const int64_t w1 = w0 + 32 < n ? w0 + 32 : n;
-        int64_t l[32] = {0};
-        int64_t total = 0;
-        for (int64_t r = w0; r < w1; ++r) {
-            const bool skip = (mask[(size_t)(w0 >> 5)] >> (r - w0)) & 1u;
-            l[r - w0] = skip ? 0 : len[r];
-            total += l[r - w0];
-        }
-        const int64_t avg = total >> 5;
-        int G = 1;
-        while (G < 32 && avg > (int64_t)G * G1_AVG) G <<= 1;
-        for (int p = 0; p < G; ++p) {
-            int64_t longest = 0;
-            for (int q = p * (32 / G); q < (p + 1) * (32 / G); ++q)
-                longest = l[q] > longest ? l[q] : longest;
-            held += 32.0 * (double)ceil_div(longest, G);
-        }
-        busy += (double)total;
-    }
-    return held > 0 ? busy / held : 1.0;
-}
-
-template <typename I>
-static int build_plan(cudaStream_t s, int64_t outer_n, int64_t nnz, const I *ptr, int base, Plan *p) {
-    std::vector<I> h((size_t)outer_n + 1);
-    int rc = check_cuda(cudaMemcpyAsync(h.data(), ptr, sizeof(I) * (outer_n + 1), cudaMemcpyDeviceToHost, s),
-                        "plan: pointer copy");
-    if (rc) return rc;
-    rc = check_cuda(cudaStreamSynchronize(s), "plan: sync");
-    if (rc) return rc;
-    std::vector<int64_t> len((size_t)outer_n);
-    int64_t maxlen = 0;
-    for (int64_t r = 0; r < outer_n; ++r) {
-        int64_t b = (int64_t)h[r] - base, e = (int64_t)h[r + 1] - base;
-        b = b < 0 ? 0 : (b > nnz ? nnz : b);
-        e = e < b ? b : (e > nnz ? nnz : e);
-        len[r] = e - b;
-        maxlen = len[r] > maxlen ? len[r] : maxlen;
-    }
-    // Natural order: a row goes to chunks when it is longer than CHUNK, or longer than
-    // PLAN_LEN and more than 4x the average of its warp's 32 rows (it would hold the
-    // warp's other rows back).  Bin order: only rows longer than CHUNK are chunked.
-    std::vector<uint32_t> mask_nat((size_t)ceil_div(outer_n, 32), 0u), mask_bin(mask_nat.size(), 0u);
-    for (int64_t w0 = 0; w0 < outer_n; w0 += 32) {
-        const int64_t w1 = w0 + 32 < outer_n ? w0 + 32 : outer_n;
-        int64_t sum = 0;
-        for (int64_t r = w0; r < w1; ++r) sum += len[r];
-        for (int64_t r = w0; r < w1; ++r) {
-            if (len[r] > CHUNK) mask_bin[(size_t)(w0 >> 5)] |= 1u << (r - w0);
-            if (len[r] > CHUNK || (len[r] > PLAN_LEN && 8 * len[r] > sum))
-                mask_nat[(size_t)(w0 >> 5)] |= 1u << (r - w0);
-        }
-    }
-    // bin order when the natural one would leave over a tenth of the lanes idle (only
-    // FP64-bound products use it, where every idle lane is lost FP64 time)
-    const bool binned = outer_n >= 32 && outer_n <= 0x7fffffffLL && natural_utilisation(len, mask_nat) < 0.9;
-    struct HostSet {
-        std::vector<int64_t> row;
-        std::vector<int32_t> first, count, slot;
-    } hs[2];
-    for (int t = 0; t < (binned ? 2 : 1); ++t) {
-        const std::vector<uint32_t> &mask = t == 0 ? mask_nat : mask_bin;
-        HostSet &h2 = hs[t];
-        for (int64_t r = 0; r < outer_n; ++r) {
-            if (!((mask[(size_t)(r >> 5)] >> (r & 31)) & 1u)) continue;
-            const int64_t nch = ceil_div(len[r], CHUNK);
-            if ((int64_t)h2.slot.size() + nch > 0x7fffffffLL)
-                return fail(GSA_ERR_UNSUPPORTED, "plan: too many chunks");
-            h2.row.push_back(r);
-            h2.first.push_back((int32_t)h2.slot.size());
-            h2.count.push_back((int32_t)nch);
-            for (int64_t q = 0; q < nch; ++q) h2.slot.push_back((int32_t)(h2.row.size() - 1));
-        }
-    }
-    std::vector<int32_t> perm, warp_group;
-    std::vector<int64_t> groups;
-    if (binned) {  // per segment, a counting sort of the unchunked rows by bin, stable
-        std::vector<int64_t> cnt(NBINS + 1);
-        for (int64_t s0 = 0; s0 < outer_n; s0 += BIN_SEGMENT) {
-            const int64_t s1 = s0 + BIN_SEGMENT < outer_n ? s0 + BIN_SEGMENT : outer_n;
-            std::fill(cnt.begin(), cnt.end(), 0);
-            for (int64_t r = s0; r < s1; ++r)
-                if (len[r] <= CHUNK) ++cnt[(size_t)bin_of(len[r]) + 1];
-            for (int b = 0; b < NBINS; ++b) cnt[(size_t)b + 1] += cnt[(size_t)b];
-            const int64_t base_pos = (int64_t)perm.size();
-            perm.resize((size_t)(base_pos + cnt[NBINS]));
-            std::vector<int64_t> at(cnt.begin(), cnt.end() - 1);
-            for (int64_t r = s0; r < s1; ++r) {
-                if (len[r] > CHUNK) continue;
-                perm[(size_t)(base_pos + at[(size_t)bin_of(len[r])]++)] = (int32_t)r;
-            }
-            // one group per lanes-per-row class: its bins are consecutive, so its rows are
-            // sorted by the work of each lane and a warp's 32 / G rows have equal or
-            // adjacent lengths (one partial warp per class and segment, not per bin)
-            for (int b0 = 0; b0 < NBINS;) {
-                const int G = bin_lanes(b0);
-                int b1 = b0;
-                while (b1 < NBINS && bin_lanes(b1) == G) ++b1;
-                const int64_t nrows = cnt[(size_t)b1] - cnt[(size_t)b0];
-                if (nrows > 0) {
-                    const int64_t nw = ceil_div(nrows, 32 / G);
-                    const int64_t gi = (int64_t)groups.size() / 4;
-                    if (gi > 0x7fffffffLL) return fail(GSA_ERR_UNSUPPORTED, "plan: too many bin groups");
-                    groups.push_back((int64_t)warp_group.size());
-                    groups.push_back(base_pos + cnt[(size_t)b0]);
-                    groups.push_back(base_pos + cnt[(size_t)b1]);
-                    groups.push_back(G);
-                    for (int64_t q = 0; q < nw; ++q) warp_group.push_back((int32_t)gi);
-                }
-                b0 = b1;
-            }
-        }
-    }
-    p->outer_n = outer_n;
-    p->nnz = nnz;
-    p->max_len = maxlen;
-    p->nbin_warps = (int64_t)warp_group.size();
-    p->nplanned = binned ? outer_n : (int64_t)hs[0].row.size();
-    if (p->nplanned == 0) return GSA_OK;
-    size_t bytes = align_up(perm.size() * 4, 256) + align_up(warp_group.size() * 4, 256) +
-                   align_up(groups.size() * 8, 256) + align_up(sizeof(gsa_bin_order), 256);
-    for (int t = 0; t < 2; ++t)
-        bytes += align_up(hs[t].row.size() * 8, 256) + align_up(hs[t].first.size() * 4, 256) +
-                 align_up(hs[t].count.size() * 4, 256) + align_up(hs[t].slot.size() * 4, 256) +
-                 align_up(mask_nat.size() * 4, 256);
-    rc = check_cuda(cudaMalloc(&p->mem, bytes), "plan: device memory");
-    if (rc) return rc;
-    Carver cv(p->mem);
-    auto up = [&](void *dst, const void *src, size_t n, const char *what) {
-        if (!rc && n) rc = check_cuda(cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice), what);
-    };
-    for (int t = 0; t < 2; ++t) {
-        gsa_chunk_set &c = t == 0 ? p->nat : p->bin;
-        const std::vector<uint32_t> &mask = t == 0 ? mask_nat : mask_bin;
-        const HostSet &h2 = hs[t];
-        int64_t *d_row = cv.take<int64_t>(h2.row.size());
-        int32_t *d_first = cv.take<int32_t>(h2.first.size());
-        int32_t *d_count = cv.take<int32_t>(h2.count.size());
-        int32_t *d_slot = cv.take<int32_t>(h2.slot.size());
-        uint32_t *d_mask = cv.take<uint32_t>(mask.size());
-        up(d_row, h2.row.data(), h2.row.size() * 8, "plan: rows");
-        up(d_first, h2.first.data(), h2.first.size() * 4, "plan: first");
-        up(d_count, h2.count.data(), h2.count.size() * 4, "plan: count");
-        up(d_slot, h2.slot.data(), h2.slot.size() * 4, "plan: chunks");
-        up(d_mask, mask.data(), mask.size() * 4, "plan: mask");
-        c.nlong = (int64_t)h2.row.size();
-        c.nchunks = (int64_t)h2.slot.size();
-        c.row = d_row;
-        c.first = d_first;
-        c.count = d_count;
-        c.chunk_slot = d_slot;
-        c.skip_mask = d_mask;
-    }
-    int32_t *d_perm = cv.take<int32_t>(perm.size());
-    int32_t *d_wg = cv.take<int32_t>(warp_group.size());
-    int64_t *d_groups = cv.take<int64_t>(groups.size());
-    up(d_perm, perm.data(), perm.size() * 4, "plan: order");
-    up(d_wg, warp_group.data(), warp_group.size() * 4, "plan: warp groups");
-    up(d_groups, groups.data(), groups.size() * 8, "plan: groups");
-    gsa_bin_order *d_view = cv.take<gsa_bin_order>(1);
-    if (binned) {
-        p->order = gsa_bin_order{p->nbin_warps, d_perm, d_wg, d_groups};
-        up(d_view, &p->order, sizeof(gsa_bin_order), "plan: bin view");
-    }
-    if (rc) return rc;
-    if (binned) p->bin_view = d_view;
-    return GSA_OK;
-}
-
-int plan_create(cudaStream_t s, int itype, int64_t outer_n, int64_t nnz, const void *ptr, int base, Plan *p) {
-    if (itype == GSA_IDX32) return build_plan<int32_t>(s, outer_n, nnz, (const int32_t *)ptr, base, p);
-    return build_plan<int64_t>(s, outer_n, nnz, (const int64_t *)ptr, base, p);
 }
 
 #define GSA_INST_RB(V, I)                                                                       \
