@@ -484,6 +484,10 @@ template <typename V, typename I>
 int launch_rowblock(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t k, DenseIn<V> B,
                     DenseOut<V> C, const Plan *plan, void *ws, size_t ws_bytes);
 size_t rowblock_workspace_size(const Plan *plan, size_t vsize, int64_t k);
+// Grouped products: one persistent launch over the tiles of a device array of items.
+template <typename V, typename I>
+int launch_grouped(cudaStream_t s, const gsa_group_item *items, int64_t count, int64_t ntiles, int base, int KC, int g1,
+                   const int32_t *tile_item);
 // Persistent bulk-copy pipelined merge-path SpMV (k = 1): GSA_ALGO_PIPE.
 template <typename V, typename I>
 int launch_spmv_pipe(cudaStream_t s, const CompressedArgs<V, I> &a, DenseIn<V> B, DenseOut<V> C,

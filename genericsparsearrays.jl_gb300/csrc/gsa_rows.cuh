@@ -77,13 +77,26 @@ __device__ __forceinline__ void accumulate_pairs(const CompressedArgs<double, I>
     for (; j < je; j += S) row_fma((O)idx[j] - base, val[j]);
 }
 
-template <typename V, typename I, int KC, int S, int U>
+// How a kernel reads B.  One of B's two strides is always one, and a kernel compiled for the
+// layout steps a pointer along a row's columns (5 instructions per entry and column); one that
+// takes both strides from B pays two 64-bit multiplies per gather (about 30).
+//   COLUMNS  column-major, all of the thread's KC columns exist: no condition stands between an
+//            entry's loads, so they are issued together (each waited for the one before where a
+//            missing column or an index outside branched around it: Float32, 16 columns on the
+//            2048^2 grid, 587 us with KC = 4; 175 us with KC = 16 this way)
+//   ROWS     row-major, columns may be missing in the last group
+//   ANY      either, columns may be missing, the shortest code: the grouped kernel, whose items
+//            differ (compiled for both layouts its registers cost more than the multiplies: 1024
+//            banded products of 1, 4 or 8 columns, Float32 600 us against 443, Float64 623 against
+//            497), and the cases that by_layout and launch_rowblock name
+enum Layout { COLUMNS, ROWS, ANY };
+
+template <typename V, typename I, int KC, int S, int U, int LAY>
 __device__ __forceinline__ void accumulate_range(const CompressedArgs<V, I> &a, const DenseIn<V> &B,
                                                  Off<I> jb, Off<I> je, int64_t c0, int64_t k,
                                                  V (&acc)[KC]) {
-    // only in the 4- and 8-column kernels (what a row-major B takes): compiled into the
-    // 2-column kernel of a column-major B it cost 8 registers and 12 % of the Laplacian SpMM
-    if constexpr (std::is_same<V, double>::value && KC >= 4) {
+    // only in the 4- and 8-column kernels (what a row-major B takes)
+    if constexpr (std::is_same<V, double>::value && KC >= 4 && LAY != COLUMNS) {
         if (B.pairs) {
             accumulate_pairs<I, KC, S, U>(a, B, jb, je, c0, k, acc);
             return;
@@ -95,6 +108,33 @@ __device__ __forceinline__ void accumulate_range(const CompressedArgs<V, I> &a, 
     const O inner = sizeof(O) == 8 ? (O)a.inner_n
                                    : (O)(a.inner_n < 0xffffffffLL ? a.inner_n : 0xffffffffLL);
     const O base = (O)a.base;
+    const V *__restrict__ p0 = B.p + (LAY == ROWS ? c0 : c0 * B.cs);
+    const int64_t rs = LAY == COLUMNS ? 1 : B.rs, step = LAY == ROWS ? 1 : B.cs;
+    auto row_mac = [&](O ci, V av) {
+        const bool ok = ci < inner;
+        // One column of one lane per row has no other load to issue, and a skipped load is the
+        // shorter code (Float64 grid SpMV 62 us against 64).
+        if constexpr (LAY == ANY || (KC == 1 && S == 1)) {
+#pragma unroll
+            for (int c = 0; c < KC; ++c)
+                if (KC == 1 || c0 + c < k) {
+                    const V xv = ok ? conj_if(ldg(p0 + (int64_t)ci * rs + c * step), B.conj) : VT<V>::zero();
+                    acc[c] = mac(acc[c], av, xv);
+                }
+        } else {  // an index outside reads row 0 and multiplies zero
+            const V *q = p0 + (int64_t)(ok ? ci : 0) * rs;
+            V x[KC];
+#pragma unroll
+            for (int c = 0; c < KC; ++c) {
+                if (KC == 1 || LAY == COLUMNS || c0 + c < k) x[c] = ldg(q);
+                q += step;
+            }
+#pragma unroll
+            for (int c = 0; c < KC; ++c)
+                if (KC == 1 || LAY == COLUMNS || c0 + c < k)
+                    acc[c] = mac(acc[c], av, ok ? conj_if(x[c], B.conj) : VT<V>::zero());
+        }
+    };
     O j = jb;
     if (U > 1) {
         for (; j + (O)((U - 1) * S) < je; j += U * S) {
@@ -106,35 +146,17 @@ __device__ __forceinline__ void accumulate_range(const CompressedArgs<V, I> &a, 
                 av[u] = conj_if(val[j + u * S], a.conjA);
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const bool ok = ci[u] < inner;
-#pragma unroll
-                for (int c = 0; c < KC; ++c)
-                    if (KC == 1 || c0 + c < k) {
-                        const V xv = ok ? B.at((int64_t)ci[u], c0 + c) : VT<V>::zero();
-                        acc[c] = mac(acc[c], av[u], xv);
-                    }
-            }
+            for (int u = 0; u < U; ++u) row_mac(ci[u], av[u]);
         }
     }
-    for (; j < je; j += S) {
-        const O c1 = (O)idx[j] - base;
-        const bool ok = c1 < inner;
-        const V av = conj_if(val[j], a.conjA);
-#pragma unroll
-        for (int c = 0; c < KC; ++c)
-            if (KC == 1 || c0 + c < k) {
-                const V xv = ok ? B.at((int64_t)c1, c0 + c) : VT<V>::zero();
-                acc[c] = mac(acc[c], av, xv);
-            }
-    }
+    for (; j < je; j += S) row_mac((O)idx[j] - base, conj_if(val[j], a.conjA));
 }
 
 // The 32 rows of one warp (lane l owns row row0 + l, entries [b, e)), G lanes per
 // row: in each of G passes the warp's 32/G groups take one row each, the group's
 // lanes stride the row, a width-G shuffle tree reduces, the group's first lane
 // stores.  G = 1 is a thread per row.
-template <typename V, typename I, int KC, int G>
+template <typename V, typename I, int KC, int G, int LAY>
 __device__ __forceinline__ void warp_rows(const CompressedArgs<V, I> &a, int64_t k, const DenseIn<V> &B,
                                           const DenseOut<V> &C, int64_t c0, int64_t row0, Off<I> b,
                                           Off<I> e, int skip) {
@@ -150,8 +172,8 @@ __device__ __forceinline__ void warp_rows(const CompressedArgs<V, I> &a, int64_t
         V acc[KC];
 #pragma unroll
         for (int c = 0; c < KC; ++c) acc[c] = VT<V>::zero();
-        accumulate_range<V, I, KC, G, (G == 1 ? GSA_G1_UNROLL : GSA_GN_UNROLL)>(a, B, qb + (O)(lane % G), qe, c0, k,
-                                                                              acc);
+        accumulate_range<V, I, KC, G, (G == 1 ? (KC >= 16 ? 2 : GSA_G1_UNROLL) : GSA_GN_UNROLL), LAY>(a, B, qb + (O)(lane % G), qe, c0,
+                                                                                  k, acc);
         if (G > 1) {
 #pragma unroll
             for (int c = 0; c < KC; ++c) {
@@ -243,7 +265,7 @@ __device__ __forceinline__ void dispatch_lanes(int64_t avg, int g1_avg, F &&f) {
 
 // One warp's 32 rows starting at row0 (a multiple of 32), G lanes per row (see
 // dispatch_lanes); rows the plan takes are left to its warps.
-template <typename V, typename I, int KC>
+template <typename V, typename I, int KC, int LAY>
 __device__ __forceinline__ void warp_unit(const CompressedArgs<V, I> &a, int64_t k, const DenseIn<V> &B,
                                           const DenseOut<V> &C, int64_t c0, int64_t row0,
                                           const uint32_t *__restrict__ skip_mask, int g1_avg = G1_AVG) {
@@ -251,7 +273,7 @@ __device__ __forceinline__ void warp_unit(const CompressedArgs<V, I> &a, int64_t
     int skip;
     const int64_t avg = warp_extent(a, row0, skip_mask, b, e, skip);
     dispatch_lanes(avg, g1_avg, [&](auto g) {
-        warp_rows<V, I, KC, decltype(g)::value>(a, k, B, C, c0, row0, b, e, skip);
+        warp_rows<V, I, KC, decltype(g)::value, LAY>(a, k, B, C, c0, row0, b, e, skip);
     });
 }
 
@@ -288,7 +310,7 @@ __device__ __forceinline__ int64_t bin_row(const CompressedArgs<V, I> &a, const 
     return row;
 }
 
-template <typename V, typename I, int KC, int G>
+template <typename V, typename I, int KC, int G, int LAY>
 __device__ __forceinline__ void binned_rows(const CompressedArgs<V, I> &a, int64_t k, const DenseIn<V> &B,
                                             const DenseOut<V> &C, int64_t c0, int64_t pos0, int64_t pend,
                                             const gsa_bin_order &bv) {
@@ -302,7 +324,7 @@ __device__ __forceinline__ void binned_rows(const CompressedArgs<V, I> &a, int64
     V acc[KC];
 #pragma unroll
     for (int c = 0; c < KC; ++c) acc[c] = VT<V>::zero();
-    accumulate_range<V, I, KC, G, 2>(a, B, b + (O)(lane % G), e, c0, k, acc);
+    accumulate_range<V, I, KC, G, 2, LAY>(a, B, b + (O)(lane % G), e, c0, k, acc);
     if (G > 1) {
 #pragma unroll
         for (int c = 0; c < KC; ++c) {
@@ -318,7 +340,7 @@ __device__ __forceinline__ void binned_rows(const CompressedArgs<V, I> &a, int64
 }
 
 // Warp w of the bin order (w < bv.nwarps).
-template <typename V, typename I, int KC>
+template <typename V, typename I, int KC, int LAY>
 __device__ __forceinline__ void binned_warp(const CompressedArgs<V, I> &a, int64_t k, const DenseIn<V> &B,
                                             const DenseOut<V> &C, int64_t c0, int64_t w,
                                             const gsa_bin_order &bv) {
@@ -326,7 +348,7 @@ __device__ __forceinline__ void binned_warp(const CompressedArgs<V, I> &a, int64
     int G;
     bin_warp(bv, w, pos0, pend, G);
     dispatch_lanes(G, 1, [&](auto g) {  // G is a power of two: picks exactly G lanes
-        binned_rows<V, I, KC, decltype(g)::value>(a, k, B, C, c0, pos0, pend, bv);
+        binned_rows<V, I, KC, decltype(g)::value, LAY>(a, k, B, C, c0, pos0, pend, bv);
     });
 }
 
