@@ -215,12 +215,13 @@ template <> __device__ __forceinline__ cf64 ld_stream(const cf64 *p) {
     return cf64{v.x, v.y};
 }
 
-// Atomic accumulate (complex: one atomic per component).
+// Atomic accumulate.  ComplexF32: both components by one vector reduction (atomic per component);
+// ComplexF64 has no such instruction and takes one atomic per component.
 __device__ __forceinline__ void atomic_add(float *p, float v) { atomicAdd(p, v); }
 __device__ __forceinline__ void atomic_add(double *p, double v) { atomicAdd(p, v); }
 __device__ __forceinline__ void atomic_add(cf32 *p, cf32 v) {
-    atomicAdd(&p->re, v.re);
-    atomicAdd(&p->im, v.im);
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(__cvta_generic_to_global(p)), "f"(v.re), "f"(v.im)
+                 : "memory");
 }
 __device__ __forceinline__ void atomic_add(cf64 *p, cf64 v) {
     atomicAdd(&p->re, v.re);

@@ -360,6 +360,25 @@ int launch_scatter(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t k, Den
     return check_cuda(cudaGetLastError(), "scatter_merge_kernel");
 }
 
+// out[key] += v for every lane with `valid`; all 32 lanes call this.
+template <typename V> __device__ __forceinline__ void add_each(V *out, int64_t key, V v, bool valid) {
+    if (valid) atomic_add(out + key, v);
+}
+// ComplexF64: neighbouring lanes exchange halves, so that one instruction adds both components of
+// the even lanes' entries and one both of the odd lanes': 16 sectors of two adds each where one
+// instruction per component touches 32 sectors with one add each.  The adds are bound by the
+// sectors that the L2's atomic units take.
+template <> __device__ __forceinline__ void add_each(cf64 *out, int64_t key, cf64 v, bool valid) {
+    const bool odd = threadIdx.x & 1;
+    const double mine = odd ? v.im : v.re, give = odd ? v.re : v.im;
+    const double got = __shfl_xor_sync(0xffffffffu, give, 1);
+    const int64_t at = valid ? key : -1, other = __shfl_xor_sync(0xffffffffu, at, 1);
+    const int64_t first = odd ? other : at, second = odd ? at : other;  // the even and the odd lane's entry
+    double *comp = reinterpret_cast<double *>(out) + odd;
+    if (first >= 0) atomicAdd(comp + 2 * first, odd ? got : mine);
+    if (second >= 0) atomicAdd(comp + 2 * second, odd ? mine : got);
+}
+
 // ---------------------------------------------------------------------------
 // COO: each warp takes 32 consecutive entries at a time; a segmented scan over runs of
 // equal adjacent output indices leaves each run's sum in its last lane, which adds it
@@ -407,8 +426,10 @@ coo_kernel(int64_t nnz, const I *__restrict__ out_idx, const I *__restrict__ in_
         // skipped (warp-uniform)
         const bool runs = __any_sync(0xffffffffu, valid && !tail);
         if (!runs) {
-            for (int64_t c = 0; c < k; ++c)
-                if (valid) atomic_add(C.p + key + c * C.ld, mul(av, xa(in, c)));
+            for (int64_t c = 0; c < k; ++c) {
+                const V v = valid ? mul(av, xa(in, c)) : VT<V>::zero();
+                add_each(C.p + c * C.ld, key, v, valid);
+            }
             continue;
         }
         int run_start = (lane == 0 || prev_key != key) ? lane : 0;
