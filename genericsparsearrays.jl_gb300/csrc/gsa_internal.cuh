@@ -298,16 +298,31 @@ __device__ __forceinline__ int64_t zero_plus(int64_t x) { return x; }
 // _rmul_or_fill!: beta == 1 keeps C, beta == 0 overwrites without reading (the
 // reference then adds into the zero it filled: 0 + t).  alpha == 1 of a real type is
 // not multiplied (t * 1 == t for every t), which saves an FP64 instruction per row.
+//
+// A ComplexF64 t times alpha = 1 + 0i is four FP64 instructions, 64 cycles of an SM's pipe for a
+// warp, and gives t's own bits unless a part of t is infinite, NaN or -0 (inf * 0 is NaN, and a -0
+// can become +0): those are multiplied, the rest is not (integer tests, off the FP64 pipe).
+__device__ __forceinline__ bool plain_part(double x) {
+    const int hi = __double2hiint(x);
+    return (hi & 0x7ff00000) != 0x7ff00000 && (hi != (int)0x80000000 || __double2loint(x) != 0);
+}
+template <typename V> __device__ __forceinline__ V times_alpha(V t, V alpha, bool one) {
+    return one ? t : mul(t, alpha);
+}
+template <> __device__ __forceinline__ cf64 times_alpha(cf64 t, cf64 alpha, bool one) {
+    return one && plain_part(t.re) && plain_part(t.im) ? t : mul(t, alpha);
+}
+
 template <typename V> struct DenseOut {
     V *p;
     int64_t ld;
     V alpha, beta;
     int beta_mode;  // 0: beta == 0, 1: beta == 1, 2: general
-    bool alpha_one; // alpha == 1 and V is real
+    bool alpha_one; // alpha == 1 and V is real, or ComplexF64 and alpha is 1 + 0i
     // C[i, c] = beta*C[i, c] + acc*alpha
     __device__ __forceinline__ void store(int64_t i, int64_t c, V acc) const {
         V *q = p + i * 1 + c * ld;
-        V t = alpha_one ? acc : mul(acc, alpha);
+        V t = times_alpha(acc, alpha, alpha_one);
         if (beta_mode == 0) *q = zero_plus(t);
         else if (beta_mode == 1) *q = add(*q, t);
         else *q = mac(t, *q, beta);
@@ -324,6 +339,11 @@ template <typename V> inline int beta_mode_of(V beta) {
 }
 template <typename V> __host__ __device__ inline bool alpha_one_of(V alpha) {
     return !VT<V>::is_complex && is_one(alpha);
+}
+template <> __host__ __device__ inline bool alpha_one_of(cf64 alpha) {  // the imaginary part +0
+    union { cf64 v; unsigned long long w[2]; } u;
+    u.v = alpha;
+    return u.w[0] == 0x3ff0000000000000ull && u.w[1] == 0ull;
 }
 
 // ---------------------------------------------------------------------------

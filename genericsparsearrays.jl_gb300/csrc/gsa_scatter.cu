@@ -124,10 +124,10 @@ scatter_merge_kernel(CompressedArgs<V, I> a, int64_t k, DenseIn<V> B, DenseOut<V
 // ---------------------------------------------------------------------------
 // Outer-block scatter (the default).
 
-// op(B)(o, c) * alpha, without the multiply when alpha == 1 of a real type (exact).
+// op(B)(o, c) * alpha.
 template <typename V>
 __device__ __forceinline__ V alpha_times(const DenseOut<V> &C, V b) {
-    return C.alpha_one ? b : mul(b, C.alpha);
+    return times_alpha(b, C.alpha, C.alpha_one);
 }
 
 // C[idx_j, c0 + c] += conj?(a_j) * xa[c] for j = jb, jb+S, ... < je; entries whose index
@@ -394,10 +394,10 @@ __global__ void __launch_bounds__(256, GSA_COO_MIN_BLOCKS)
 coo_kernel(int64_t nnz, const I *__restrict__ out_idx, const I *__restrict__ in_idx,
            const V *__restrict__ val, int base, bool conjA, int64_t k, DenseIn<V> B,
            DenseOut<V> C, int64_t out_rows, int64_t in_rows) {
-    // op(B)(in, c) * alpha (alpha == 1 of a real type needs no multiply: exact)
+    // op(B)(in, c) * alpha
     auto xa = [&](int64_t in, int64_t c) -> V {
         const V x = B.at(in, c);
-        return C.alpha_one ? x : mul(x, C.alpha);
+        return times_alpha(x, C.alpha, C.alpha_one);
     };
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;

@@ -43,3 +43,24 @@ def test_no_columns(gsa, cuda, k):
         C = torch.ones((k, 3), dtype=torch.from_numpy(np.zeros(1, dt)).dtype, device=cuda).t()
         gsa.mul_(C, A, torch.empty((k, 0), dtype=C.dtype, device=cuda).t(), 1, 2)
         assert np.array_equal(C.cpu().numpy(), np.full((3, k), 2, dt))
+
+
+@pytest.mark.parametrize("fmt", ["csr", "csc", "coo"])
+@pytest.mark.parametrize("k", [1, 3])
+def test_complex_alpha_one_keeps_special_values(gsa, cuda, fmt, k):
+    """alpha = 1 + 0i is not multiplied where that changes no bit; infinities, NaN and -0 come out as
+    the product with alpha gives them: as alpha = 2 + 0i gives them, halved."""
+    s = np.array([0.0, -0.0, 1.5, -2.25, np.inf, -np.inf, np.nan])
+    x = np.empty((7, 7), np.complex128)
+    x.real, x.imag = np.meshgrid(s, s)
+    x = np.repeat(x.reshape(-1, 1), k, 1)
+    n = x.shape[0]
+    p = np.random.default_rng(0).permutation(n) if fmt == "coo" else np.arange(n)
+    eye = np.arange(1, n + 1)
+    cls = {"csr": gsa.GenericSparseMatrixCSR, "csc": gsa.GenericSparseMatrixCSC, "coo": gsa.GenericSparseMatrixCOO}[fmt]
+    ptr = eye[p] if fmt == "coo" else np.arange(1, n + 2)
+    A = gsa.adapt(cuda, cls(n, n, ptr, eye[p], np.ones(n, np.complex128)))
+    X = torch.from_numpy(np.asfortranarray(x)).to(cuda)
+    one, two = (gsa.mul_(torch.zeros_like(X), A, X, al, 0).cpu().numpy().copy().view(np.float64) for al in (1, 2))
+    assert np.array_equal(one, two / 2, equal_nan=True)
+    assert np.array_equal(np.signbit(one) & ~np.isnan(one), np.signbit(two) & ~np.isnan(two))
