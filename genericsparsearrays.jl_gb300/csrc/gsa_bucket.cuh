@@ -16,16 +16,16 @@
 //      record: the key row-in-bucket << (mb + pb) | minor << pb | position (sorting a row by it
 //      is sorting by (minor, position)) and the value (conversions), one 16- or 32-byte store.
 //   C. fine_kernel: a CTA per coarse bucket counts its rows in shared memory, scans them --
-//      the row pointers of the result -- and places the bucket's entries in row order into
-//      shared memory (96 KB of staging; cs is chosen so that an average bucket fills at most
-//      half of it).  Rows of up to 16 entries are sorted there by a thread in registers (rank
-//      counting), rows of up to 256 by a warp, and emitted; longer rows go to cta_kernel
-//      (rank counting up to 1024 entries, else a bitonic sort of 16384-entry chunks in shared
-//      memory, merged pairwise; values then gathered by input position).  A bucket larger than the staging is placed in global
-//      memory instead, with its rows of more than 16 entries listed for warp_kernel and
-//      cta_kernel.  Where rows average at most 8 entries, fine_stage_kernel runs this pass
-//      instead: one CTA per SM, the next bucket's records copied into shared memory while the
-//      current one is sorted, the bucket's output written with coalesced stores.
+//      the row pointers of the result -- and places the bucket's keys in row order into shared
+//      memory (cs is chosen so that an average bucket fills at most half of the staging).  Every
+//      entry of a row of up to 256 counts the row's smaller keys and writes itself to its place.
+//      Longer rows go to the kernels of longer rows: chunks of 4096 entries sorted by a CTA each,
+//      then merged by counting (values gathered by input position).  A bucket larger than the
+//      staging is placed in global memory instead, its rows of up to 16 entries sorted by a
+//      thread, up to 256 by a warp (warp_kernel).  Where rows average at most 8 entries,
+//      fine_stage_kernel runs this pass instead: one CTA per SM, the next bucket's records copied
+//      into shared memory while the current one is sorted, the bucket's output written with
+//      coalesced stores.
 // Matrices with more than 8191 x 4096 rows take the one-level form (count, place, and
 // small_kernel per row), whose stores are random.
 //
@@ -48,11 +48,9 @@ namespace bucket {
 
 constexpr int SMALL = 16;          // a thread sorts rows of up to 16 entries in registers
 constexpr int WARP_MAX = 256;      // a warp sorts rows of up to 256 entries
-constexpr int CTA_THREADS = 1024;
-constexpr int CTA_TILE = 16384;    // a CTA sorts 16384 entries in shared memory at once (128 KB)
-constexpr int RANK_MAX = 1024;     // a CTA ranks rows of up to 1024 entries by counting
+constexpr int LONG_THREADS = 512;
+constexpr int LONG_CHUNK = 4096;   // entries of a longer row that a CTA sorts in shared memory (32 KB)
 constexpr int WARP_CTA_THREADS = 256;
-constexpr int MERGE_ITEMS = 8;
 constexpr int ROWS_MAX = 4096;     // rows per coarse bucket
 constexpr int COARSE_MAX = 8192;   // coarse buckets, the invalid-row bucket included
 constexpr int PB_THREADS = 256, PB_ITEMS = 8;
@@ -157,7 +155,7 @@ template <class Emit> struct PackedEmit {
 struct Layout {
     Coarse co;
     int64_t ncnt;
-    size_t cnt, cstart, start, bsums, key1, rec1, key2, val2, list, counters, bytes;
+    size_t cnt, cstart, start, bsums, key1, rec1, key2, val2, list, items, counters, bytes;
 };
 
 // vsize: bytes of a carried value (0: none)
@@ -172,11 +170,12 @@ inline Layout layout(int64_t major_n, int64_t minor_n, int64_t nnz, size_t vsize
     L.cstart = cv.reserve<uint32_t>(L.ncnt);
     L.start = cv.reserve<uint32_t>(major_n + 2);
     L.bsums = cv.reserve<uint32_t>(ceil_div(nscan, (int64_t)sc_tile) + 1);
-    L.key1 = cv.reserve<uint64_t>(n);
-    L.key2 = cv.reserve<uint64_t>(n);
+    L.key1 = L.co.ok ? 0 : cv.reserve<uint64_t>(n);
+    L.key2 = L.co.ok ? cv.reserve<uint64_t>(n) : 0;
     L.rec1 = L.co.ok ? cv.reserve<unsigned char>((size_t)n * rec_size(vsize)) : 0;
     L.val2 = L.co.ok && vsize ? cv.reserve<unsigned char>((size_t)n * vsize) : 0;
     L.list = cv.reserve<uint32_t>(major_n + 1);
+    L.items = cv.reserve<uint2>(n / WARP_MAX + n / LONG_CHUNK + 1);
     L.counters = cv.reserve<uint32_t>(4);
     L.bytes = align_up(cv.off, 256);
     return L;
@@ -226,22 +225,35 @@ __device__ __forceinline__ void sort_short_row(const uint64_t *keys, const VT *v
     else if (len <= SMALL) sort_registers<Emit, VT, SMALL>(keys, vals, out, len, r, emit);
 }
 
-// Rows longer than SMALL go to the lists: warp-sized from the front, CTA-sized from the
-// back (one atomic per warp and list).  All 32 lanes call this.
-__device__ __forceinline__ void list_long_rows(bool valid, uint32_t len, uint32_t r, int64_t major_n,
-                                               uint32_t *list, uint32_t *counters) {
+// What is left for the kernels of longer rows: rows of (SMALL, WARP_MAX] entries (list, counted
+// in counters[0]) and the chunks of LONG_CHUNK entries of still longer ones (items: row, chunk;
+// counters[1]).
+struct LongRows {
+    uint32_t *list;
+    uint2 *items;
+    uint32_t *counters;
+};
+// One atomic per warp and kind.  All 32 lanes call this.
+__device__ __forceinline__ void list_long_rows(bool valid, uint32_t len, uint32_t r, const LongRows &L) {
     const bool to_warp = valid && len > SMALL && len <= WARP_MAX;
-    const bool to_cta = valid && len > WARP_MAX;
-    const unsigned mw = __ballot_sync(0xffffffffu, to_warp), mc = __ballot_sync(0xffffffffu, to_cta);
+    const bool to_items = valid && len > WARP_MAX;
+    const unsigned mw = __ballot_sync(0xffffffffu, to_warp), mi = __ballot_sync(0xffffffffu, to_items);
     const int lane = threadIdx.x & 31;
-    const unsigned lt = lanemask_lt();
-    uint32_t bw = 0, bc = 0;
-    if (lane == 0 && mw) bw = atomicAdd(&counters[0], (uint32_t)__popc(mw));
-    if (lane == 0 && mc) bc = atomicAdd(&counters[1], (uint32_t)__popc(mc));
-    bw = __shfl_sync(0xffffffffu, bw, 0);
-    bc = __shfl_sync(0xffffffffu, bc, 0);
-    if (to_warp) list[bw + __popc(mw & lt)] = r;
-    if (to_cta) list[major_n - (bc + __popc(mc & lt))] = r;
+    if (mw) {
+        uint32_t b = 0;
+        if (lane == 0) b = atomicAdd(&L.counters[0], (uint32_t)__popc(mw));
+        b = __shfl_sync(0xffffffffu, b, 0);
+        if (to_warp) L.list[b + __popc(mw & lanemask_lt())] = r;
+    }
+    for (unsigned todo = mi; todo; todo &= todo - 1) {  // a row's chunks, by the whole warp
+        const int l = __ffs(todo) - 1;
+        const uint32_t n = (__shfl_sync(0xffffffffu, len, l) - 1) / LONG_CHUNK + 1;
+        const uint32_t row = __shfl_sync(0xffffffffu, r, l);
+        uint32_t b = 0;
+        if (lane == 0) b = atomicAdd(&L.counters[1], n);
+        b = __shfl_sync(0xffffffffu, b, 0);
+        for (uint32_t q = lane; q < n; q += 32) L.items[b + q] = make_uint2(row, q);
+    }
 }
 
 // ---- two-level form --------------------------------------------------------
@@ -349,40 +361,48 @@ coarse_place_kernel(Src src, const VT *__restrict__ vals_in, int64_t nnz, int64_
     }
 }
 
-// Dynamic shared memory of fine_kernel: the staged keys and values, then row offsets and
-// fill counters for 2^cs rows.
+// Dynamic shared memory of fine_kernel: the staged keys, row offsets and fill counters for 2^cs
+// rows, and (with values) the record of each key.
 template <class VT> inline size_t fine_smem_bytes(int cs) {
-    return (size_t)stage_entries<VT>() * (8 + carried_size<VT>()) + (((size_t)2 << cs) + 2) * sizeof(uint32_t);
+    return (size_t)stage_entries<VT>() * (8 + (carried_size<VT>() ? 2 : 0)) + (((size_t)2 << cs) + 2) * sizeof(uint32_t);
 }
 
-// CTA per coarse bucket: rows counted and scanned in shared memory (the row pointers), then
-// the bucket's entries placed in row order -- into shared memory when the bucket fits the
-// staging (rows of up to 16 entries sorted there by a thread, up to 256 by a warp, longer
-// ones copied out for cta_kernel), else into key2 / val2 (read back in this kernel: plain
-// pointers, no read-only cache path) with rows of more than 16 entries listed for
-// warp_kernel and cta_kernel.
+// CTA per coarse bucket, taken from a queue (counters[2]): rows counted and scanned in shared
+// memory (the row pointers), then the bucket's keys placed in row order -- into shared memory when
+// the bucket fits the staging, else into key2 / val2 (read back in this kernel: plain pointers, no
+// read-only cache path) with rows of more than 16 entries listed for the kernels of longer rows.
+//
+// Staged, every entry of a row of up to 256 finds its place by counting the row's smaller keys, a
+// thread per entry whatever its row: consecutive threads hold the entries of a row, so their reads
+// of its keys are broadcasts and their outputs one stretch, and no warp is left with a long row of
+// its own.  (A thread per row of up to 16 entries and a warp per longer one took 640 us for the
+// power-law ComplexF64 matrix, 16.4M entries in 10^6 rows, against 395: most of a bucket's time went
+// to the warp that had its longest row.  The COO sum's 42M keys: 490 against 289 us.  Three or four
+// CTAs per SM make no difference.)  Values stay in the bucket's records, in L2, until they are written.
+// Longer rows are copied out for the kernels of longer rows.
 template <class VT, class Emit>
 __global__ void __launch_bounds__(PC_THREADS, 2)
 fine_kernel(int64_t major_n, Coarse co, const uint32_t *__restrict__ cstart, const Rec<VT> *__restrict__ rec1,
-            uint64_t *key2, VT *val2, uint32_t *__restrict__ start, uint32_t *__restrict__ list,
-            uint32_t *__restrict__ counters, Emit emit) {
+            uint64_t *key2, VT *val2, uint32_t *__restrict__ start, LongRows longs, Emit emit) {
     constexpr bool HAS_VAL = !std::is_same<VT, NoValue>::value;
     const int cs = co.cs;
     const int64_t nb = co.nb;
     const int rshift = co.mb + co.pb;  // the row inside the bucket sits above minor and position
     const PackedEmit<Emit> pemit{emit, co.mb, co.pb};
     constexpr int STAGE = stage_entries<VT>();
+    static_assert(STAGE <= 65536, "16-bit record numbers");
     constexpr int ITEMS = ROWS_MAX / PC_THREADS;
     extern __shared__ __align__(16) unsigned char dsm[];
     uint64_t *s_key = (uint64_t *)dsm;
-    VT *s_val = (VT *)(dsm + (size_t)STAGE * 8);
-    uint32_t *s_off = (uint32_t *)(dsm + (size_t)STAGE * (8 + carried_size<VT>()));
+    uint32_t *s_off = (uint32_t *)(s_key + STAGE);
     const int rmax = 1 << cs;
-    uint32_t *s_fill = s_off + rmax + 1;  // counts, then fill cursors, then the warp row list
+    uint32_t *s_fill = s_off + rmax + 1;  // counts, then fill cursors
+    uint16_t *s_src = (uint16_t *)(s_fill + rmax + 1);
     __shared__ uint32_t s_warp[PC_THREADS / 32];
-    __shared__ uint32_t s_nlist, s_long;
+    __shared__ uint32_t s_long;
+    __shared__ int64_t s_next;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int64_t bk = blockIdx.x; bk < nb; bk += gridDim.x) {
+    for (int64_t bk = blockIdx.x; bk < nb;) {
         const uint32_t B0 = cstart[bk], B1 = cstart[bk + 1];
         const uint32_t E = B1 - B0;
         const bool invalid = bk == nb - 1;
@@ -392,7 +412,7 @@ fine_kernel(int64_t major_n, Coarse co, const uint32_t *__restrict__ cstart, con
         const bool staged = E <= (uint32_t)STAGE;
         for (int j = threadIdx.x; j < R; j += PC_THREADS) s_fill[j] = 0;
         if (threadIdx.x == 0) {
-            s_nlist = 0;
+            s_next = (int64_t)gridDim.x + atomicAdd(&longs.counters[2], 1u);
             s_long = 0;
         }
         __syncthreads();
@@ -416,80 +436,62 @@ fine_kernel(int64_t major_n, Coarse co, const uint32_t *__restrict__ cstart, con
         }
         if (lane == 31) s_warp[warp] = x;
         __syncthreads();
-        if (warp == 0) {
-            uint32_t wsum = lane < PC_THREADS / 32 ? s_warp[lane] : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, wsum, o);
-                if (lane >= o) wsum += y;
-            }
-            if (lane < PC_THREADS / 32) s_warp[lane] = wsum;
-        }
-        __syncthreads();
-        uint32_t run = (warp ? s_warp[warp - 1] : 0) + x - sum;
+        uint32_t run = x - sum;
+        for (int w = 0; w < warp; ++w) run += s_warp[w];
 #pragma unroll
         for (int q = 0; q < ITEMS; ++q) {
             const int j = threadIdx.x * ITEMS + q;
-            if (j < R) s_off[j] = run;
+            if (j < R) {
+                s_off[j] = run;
+                s_fill[j] = run;  // the row's fill cursor
+                const uint32_t first = B0 + run;
+                start[row0 + j] = first;
+                emit.pointer(row0 + j, first);
+                if (v[q] > (uint32_t)WARP_MAX) s_long = 1;
+            }
             run += v[q];
         }
         if (threadIdx.x == 0) s_off[R] = E;
-        __syncthreads();
-        for (int j = threadIdx.x; j < R; j += PC_THREADS) {
-            const uint32_t first = B0 + s_off[j];
-            start[row0 + j] = first;
-            emit.pointer(row0 + j, first);
-            s_fill[j] = 0;
-            if (s_off[j + 1] - s_off[j] > (uint32_t)WARP_MAX) s_long = 1;
-        }
         if (invalid && threadIdx.x == 0) start[major_n + 1] = B1;
         __syncthreads();
         if (staged) {
 #pragma unroll 4
-            for (uint32_t i = B0 + threadIdx.x; i < B1; i += PC_THREADS) {
-                const Rec<VT> r = rec1[i];
-                const uint32_t row = (uint32_t)shr64(r.key, rshift);
-                const uint32_t slot = s_off[row] + atomicAdd(&s_fill[row], 1u);
-                s_key[slot] = r.key;
-                if constexpr (HAS_VAL) s_val[slot] = r.val;
+            for (uint32_t i = threadIdx.x; i < E; i += PC_THREADS) {
+                const uint64_t k = rec1[B0 + i].key;
+                const uint32_t slot = atomicAdd(&s_fill[(uint32_t)shr64(k, rshift)], 1u);
+                s_key[slot] = k;
+                if constexpr (HAS_VAL) s_src[slot] = (uint16_t)i;
             }
             __syncthreads();
-            if (s_long) {  // rows for cta_kernel read their (plain) keys from key2
-                for (uint32_t j = threadIdx.x; j < E; j += PC_THREADS)
-                    key2[B0 + j] = canonical_key(s_key[j], co.mb, co.pb);
-            }
-            __syncthreads();  // s_fill becomes the list of warp-sized rows
-            for (int j0 = 0; j0 < R; j0 += PC_THREADS) {
-                const int j = j0 + threadIdx.x;
-                const bool valid = j < R;
-                uint32_t len = 0;
-                if (valid) {
-                    len = s_off[j + 1] - s_off[j];
-                    if (len <= (uint32_t)SMALL)
-                        sort_short_row(s_key + s_off[j], HAS_VAL ? s_val + s_off[j] : nullptr, B0 + s_off[j], len,
-                                       (uint64_t)(row0 + j), pemit);
-                    else if (len <= (uint32_t)WARP_MAX)
-                        s_fill[atomicAdd(&s_nlist, 1u)] = (uint32_t)j;
+            for (uint32_t p = threadIdx.x; p < E; p += PC_THREADS) {
+                const uint64_t k = s_key[p];
+                const uint32_t row = (uint32_t)shr64(k, rshift);
+                const uint32_t o = s_off[row], len = s_off[row + 1] - o;
+                if (len > (uint32_t)WARP_MAX) {  // read back (as plain keys) by the kernels of longer rows
+                    key2[B0 + p] = canonical_key(k, co.mb, co.pb);
+                    continue;
                 }
-                list_long_rows(valid && len > (uint32_t)WARP_MAX, len, (uint32_t)(row0 + j), major_n, list,
-                               counters);
+                VT val;
+                if constexpr (HAS_VAL) val = rec1[B0 + s_src[p]].val;
+                uint32_t rank = 0;
+                const uint64_t *sk = s_key + o;
+#pragma unroll 4
+                for (uint32_t u = 0; u < len; ++u) rank += sk[u] < k ? 1u : 0u;
+                const uint32_t at = B0 + o + rank;
+                if constexpr (HAS_VAL) pemit.put(at, (uint64_t)(row0 + row), k, val);
+                else pemit.gather(at, (uint64_t)(row0 + row), k);
             }
-            __syncthreads();
-            for (uint32_t q = warp; q < s_nlist; q += PC_THREADS / 32) {
-                const uint32_t j = s_fill[q];
-                const uint32_t o = s_off[j], len = s_off[j + 1] - o;
-                for (uint32_t t = lane; t < len; t += 32) {
-                    const uint64_t kt = s_key[o + t];
-                    uint32_t rank = 0;
-                    for (uint32_t u = 0; u < len; ++u) rank += s_key[o + u] < kt ? 1u : 0u;
-                    emit_one(pemit, B0 + o + rank, (uint64_t)(row0 + j), kt, HAS_VAL ? s_val + o : nullptr, t);
+            if (s_long) {  // uniform
+                for (int j0 = 0; j0 < R; j0 += PC_THREADS) {
+                    const int j = j0 + threadIdx.x;
+                    const uint32_t len = j < R ? s_off[j + 1] - s_off[j] : 0u;
+                    list_long_rows(len > (uint32_t)WARP_MAX, len, (uint32_t)(row0 + j), longs);
                 }
             }
         } else {
             for (uint32_t i = B0 + threadIdx.x; i < B1; i += PC_THREADS) {
                 const Rec<VT> r = rec1[i];
-                const uint32_t row = (uint32_t)shr64(r.key, rshift);
-                const uint32_t slot = B0 + s_off[row] + atomicAdd(&s_fill[row], 1u);
+                const uint32_t slot = B0 + atomicAdd(&s_fill[(uint32_t)shr64(r.key, rshift)], 1u);
                 key2[slot] = canonical_key(r.key, co.mb, co.pb);
                 if constexpr (HAS_VAL) val2[slot] = r.val;
             }
@@ -504,10 +506,12 @@ fine_kernel(int64_t major_n, Coarse co, const uint32_t *__restrict__ cstart, con
                     if (len <= (uint32_t)SMALL)
                         sort_short_row(key2 + b, HAS_VAL ? val2 + b : nullptr, b, len, (uint64_t)(row0 + j), emit);
                 }
-                list_long_rows(valid, len, (uint32_t)(row0 + j), major_n, list, counters);
+                list_long_rows(valid, len, (uint32_t)(row0 + j), longs);
             }
         }
         __syncthreads();
+        bk = s_next;
+        __syncthreads();  // s_next is written again at the top
     }
 }
 
@@ -616,14 +620,14 @@ template <class VT> inline size_t fine_stage_smem(int cs, int cap) {
 // Pass C, staged: one CTA per SM takes buckets from a queue (counters[2]) and copies the
 // next bucket's records into shared memory while it sorts the current one.  Rows are
 // counted, scanned (the row pointers) and placed as record indices; rows of up to 16
-// entries are sorted by a thread, up to 256 by a warp, longer ones listed for cta_kernel;
+// entries are sorted by a thread, up to 256 by a warp, longer ones listed for the kernels of longer rows;
 // then the bucket's output is written in order.  A bucket of more than `cap` entries takes
 // fine_kernel's global path (rows placed into key2 / val2, then sorted there or listed).
 template <class VT, class Emit>
 __global__ void __launch_bounds__(ST_THREADS, 1)
 fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restrict__ cstart,
                   const Rec<VT> *__restrict__ rec1, uint64_t *key2, VT *val2, uint32_t *__restrict__ start,
-                  uint32_t *__restrict__ list, uint32_t *__restrict__ counters, Emit emit) {
+                  LongRows longs, Emit emit) {
     constexpr bool HAS_VAL = !std::is_same<VT, NoValue>::value;
     constexpr int ITEMS = ROWS_MAX / ST_THREADS;
     const int cs = co.cs;
@@ -656,7 +660,7 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
         const bool staged = E <= (uint32_t)cap;
         for (int j = threadIdx.x; j < R; j += ST_THREADS) s_cnt[j] = 0;
         if (threadIdx.x == 0) {
-            s_next = (int64_t)gridDim.x + atomicAdd(&counters[2], 1u);
+            s_next = (int64_t)gridDim.x + atomicAdd(&longs.counters[2], 1u);
             s_nlist = 0;
             s_long = 0;
         }
@@ -740,7 +744,7 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
                 if (j < E) s_idx[s_off[pr[q] >> 16] + (pr[q] & 0xffffu)] = (uint16_t)j;
             }
             __syncthreads();
-            if (s_long) {  // rows for cta_kernel read their (plain) keys from key2
+            if (s_long) {  // longer rows are read back as plain keys
                 for (uint32_t p = threadIdx.x; p < E; p += ST_THREADS)
                     key2[B0 + p] = canonical_key(s_rec[s_idx[p]].key, co.mb, co.pb);
             }
@@ -754,8 +758,7 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
                     if (len <= (uint32_t)STAGE_SMALL) sort_idx_short(s_rec, s_idx + o, len);
                     else if (len <= (uint32_t)WARP_MAX) s_cnt[atomicAdd(&s_nlist, 1u)] = (uint32_t)j;
                 }
-                list_long_rows(valid && len > (uint32_t)WARP_MAX, len, (uint32_t)(row0 + j), major_n, list,
-                               counters);
+                list_long_rows(valid && len > (uint32_t)WARP_MAX, len, (uint32_t)(row0 + j), longs);
             }
             __syncthreads();
             if (s_nlist) {  // uniform
@@ -766,7 +769,7 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
                 }
                 __syncthreads();
             }
-            // the bucket's output in order (rows listed for cta_kernel are rewritten by it)
+            // the bucket's output in order (longer rows are rewritten by their kernels)
             for (uint32_t p = threadIdx.x; p < E; p += ST_THREADS) {
                 const Rec<VT> r = s_rec[s_idx[p]];
                 const uint64_t row = (uint64_t)row0 + shr64(r.key, rshift);
@@ -793,7 +796,7 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
                     if (len <= (uint32_t)SMALL)
                         sort_short_row(key2 + b2, HAS_VAL ? val2 + b2 : nullptr, b2, len, (uint64_t)(row0 + j), emit);
                 }
-                list_long_rows(valid, len, (uint32_t)(row0 + j), major_n, list, counters);
+                list_long_rows(valid, len, (uint32_t)(row0 + j), longs);
             }
         }
         __syncthreads();
@@ -825,7 +828,7 @@ __global__ void place_kernel(Src src, int64_t nnz, int64_t major_n, const uint32
 
 template <class Emit>
 __global__ void small_kernel(int64_t major_n, const uint32_t *__restrict__ start, const uint64_t *__restrict__ keys,
-                             uint32_t *__restrict__ list, uint32_t *__restrict__ counters, Emit emit) {
+                             LongRows longs, Emit emit) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x; r0 <= major_n; r0 += stride) {
         const int64_t r = r0 + threadIdx.x;
@@ -837,7 +840,7 @@ __global__ void small_kernel(int64_t major_n, const uint32_t *__restrict__ start
             emit.pointer(r, b);
             if (len <= (uint32_t)SMALL) sort_short_row<Emit, NoValue>(keys + b, nullptr, b, len, (uint64_t)r, emit);
         }
-        list_long_rows(valid, len, (uint32_t)r, major_n, list, counters);
+        list_long_rows(valid, len, (uint32_t)r, longs);
     }
 }
 
@@ -848,13 +851,13 @@ __global__ void small_kernel(int64_t major_n, const uint32_t *__restrict__ start
 template <class VT, class Emit>
 __global__ void __launch_bounds__(WARP_CTA_THREADS)
 warp_kernel(const uint32_t *__restrict__ start, const uint64_t *__restrict__ keys, const VT *__restrict__ vals,
-            const uint32_t *__restrict__ list, const uint32_t *__restrict__ counters, Emit emit) {
+            LongRows longs, Emit emit) {
     __shared__ uint64_t s[WARP_CTA_THREADS / 32][WARP_MAX];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t nlisted = counters[0];
+    const uint32_t nlisted = longs.counters[0];
     const int64_t warps = (int64_t)gridDim.x * (WARP_CTA_THREADS / 32);
     for (int64_t q = (int64_t)blockIdx.x * (WARP_CTA_THREADS / 32) + w; q < nlisted; q += warps) {
-        const uint32_t r = list[q];
+        const uint32_t r = longs.list[q];
         const uint32_t b = start[r], len = start[r + 1] - b;
         for (uint32_t j = lane; j < len; j += 32) s[w][j] = keys[b + j];
         __syncwarp();
@@ -868,113 +871,124 @@ warp_kernel(const uint32_t *__restrict__ start, const uint64_t *__restrict__ key
     }
 }
 
+// Bitonic sort of s[0 .. P), P a power of two of at least 32, by the CTA.  Distances below 32 are
+// exchanged by shuffles (element i is in lane i mod 32 of whichever warp holds it), one pass and
+// barrier for all of a stage's: 36 barriers for 4096 keys instead of 78.
 __device__ __forceinline__ void bitonic_shared(uint64_t *s, uint32_t P) {
-    for (uint32_t k = 2; k <= P; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
-                const uint32_t ixj = i ^ j;
-                if (ixj > i) {
-                    const uint64_t a = s[i], c = s[ixj];
-                    const bool up = (i & k) == 0;
-                    if ((a > c) == up) {
-                        s[i] = c;
-                        s[ixj] = a;
-                    }
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t k = 32; k <= P; k <<= 1) {
+        for (uint32_t j = k >> 1; j >= 32; j >>= 1) {
+            for (uint32_t t = threadIdx.x; t < P / 2; t += blockDim.x) {
+                const uint32_t i = 2 * t - (t & (j - 1));
+                const uint64_t a = s[i], c = s[i + j];
+                if ((a > c) == ((i & k) == 0)) {
+                    s[i] = c;
+                    s[i + j] = a;
                 }
             }
             __syncthreads();
         }
+        for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {  // whole warps: P is a multiple of 32
+            uint64_t x = s[i];
+            // the first pass sorts every 32 keys from scratch
+            for (uint32_t kk = k == 32 ? 2 : k; kk <= k; kk <<= 1) {
+                const bool up = (i & kk) == 0;
+                for (uint32_t j = kk >> 1 < 16 ? kk >> 1 : 16; j > 0; j >>= 1) {
+                    const uint64_t y = __shfl_xor_sync(0xffffffffu, x, j);
+                    const bool low = (lane & j) == 0;
+                    x = (x < y) == (low == up) ? x : y;
+                }
+            }
+            s[i] = x;
+        }
+        __syncthreads();
     }
 }
 
-// One CTA merges the sorted runs A (na) and B (nb) into out (distinct keys).
-__device__ __forceinline__ void merge_runs(const uint64_t *A, uint32_t na, const uint64_t *B, uint32_t nb,
-                                           uint64_t *out) {
-    const uint32_t total = na + nb;
-    for (uint32_t t0 = 0; t0 < total; t0 += blockDim.x * MERGE_ITEMS) {
-        const uint32_t d0 = t0 + threadIdx.x * MERGE_ITEMS;
-        if (d0 >= total) continue;
-        uint32_t lo = d0 > nb ? d0 - nb : 0, hi = d0 < na ? d0 : na;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (A[mid] < B[d0 - 1 - mid]) lo = mid + 1;
-            else hi = mid;
-        }
-        uint32_t i = lo, j = d0 - lo;
-        for (int q = 0; q < MERGE_ITEMS && d0 + q < total; ++q) {
-            if (j >= nb || (i < na && A[i] < B[j])) out[d0 + q] = A[i++];
-            else out[d0 + q] = B[j++];
-        }
-    }
-}
-
-// CTA per listed row of more than WARP_MAX entries.  Rows of up to RANK_MAX keys: each key's
-// position is the number of smaller keys in the row (shared memory, two barriers per row);
-// up to CTA_TILE keys: bitonic sort in shared memory; longer rows sorted in CTA_TILE chunks,
-// then merged pairwise between keys and scratch (the row's own range in each).  Values are
-// gathered by input position.
+// Rows of more than WARP_MAX entries, in two kernels, a CTA per listed chunk of LONG_CHUNK entries.
+// long_sort_kernel sorts a chunk in shared memory and writes the row if that is all of it;
+// long_merge_kernel gives every entry of a row of several chunks its place: its own in its chunk
+// plus, for each other chunk (read into shared memory in turn), the number of smaller keys there.
+// Keys are distinct (they hold the input position).  Values are gathered by input position.
+//
+// A row's chunks are spread over the SMs, so the longest row sets no tail: one CTA per row, chunk
+// sorts, pairwise merges and all, took 1.0 to 1.2 ms for the power-law matrix of 10^6 rows, one SM
+// busy with its row of 50,000 entries all that time, against 0.2 (sort) and 0.1 ms (merge).  The work of a row grows with the square of
+// its chunks, and stays below the pairwise merges' up to rows of some 10^8 entries.
 template <class Emit>
-__global__ void __launch_bounds__(CTA_THREADS)
-cta_kernel(int64_t major_n, const uint32_t *__restrict__ start, uint64_t *keys, uint64_t *scratch,
-           const uint32_t *__restrict__ list, const uint32_t *__restrict__ counters, Emit emit) {
-    extern __shared__ __align__(16) uint64_t s[];  // CTA_TILE keys
-    const uint32_t nlisted = counters[1];
-    for (uint32_t q = blockIdx.x; q < nlisted; q += gridDim.x) {
-        const uint32_t r = list[major_n - q];
-        const uint32_t b = start[r], len = start[r + 1] - b;
-        if (len <= (uint32_t)RANK_MAX) {  // keys are distinct (they hold the input position)
-            for (uint32_t j = threadIdx.x; j < len; j += blockDim.x) s[j] = keys[b + j];
-            __syncthreads();
-            for (uint32_t j = threadIdx.x; j < len; j += blockDim.x) {
-                const uint64_t kj = s[j];
-                uint32_t rank = 0;
-#pragma unroll 4
-                for (uint32_t u = 0; u < len; ++u) rank += s[u] < kj ? 1u : 0u;
-                emit.gather(b + rank, (uint64_t)r, kj);
-            }
-            __syncthreads();
-            continue;
+__global__ void __launch_bounds__(LONG_THREADS)
+long_sort_kernel(const uint32_t *__restrict__ start, uint64_t *keys, LongRows longs, Emit emit) {
+    __shared__ uint64_t s[LONG_CHUNK];
+    const uint32_t nitems = longs.counters[1];
+    for (uint32_t q = blockIdx.x; q < nitems; q += gridDim.x) {
+        const uint2 item = longs.items[q];
+        const uint32_t b = start[item.x], len = start[item.x + 1] - b, c0 = item.y * LONG_CHUNK;
+        const uint32_t n = len - c0 < (uint32_t)LONG_CHUNK ? len - c0 : (uint32_t)LONG_CHUNK;
+        uint32_t P = 32;
+        while (P < n) P <<= 1;
+        for (uint32_t j = threadIdx.x; j < P; j += LONG_THREADS) s[j] = j < n ? keys[b + c0 + j] : ~0ull;
+        __syncthreads();
+        bitonic_shared(s, P);
+        for (uint32_t j = threadIdx.x; j < n; j += LONG_THREADS) {
+            if (len <= (uint32_t)LONG_CHUNK) emit.gather(b + j, (uint64_t)item.x, s[j]);
+            else keys[b + c0 + j] = s[j];
         }
-        for (uint32_t c0 = 0; c0 < len; c0 += CTA_TILE) {
-            const uint32_t n = len - c0 < (uint32_t)CTA_TILE ? len - c0 : (uint32_t)CTA_TILE;
-            uint32_t P = 2;
-            while (P < n) P <<= 1;
-            for (uint32_t j = threadIdx.x; j < P; j += blockDim.x) s[j] = j < n ? keys[b + c0 + j] : ~0ull;
-            __syncthreads();
-            bitonic_shared(s, P);
-            if (len <= (uint32_t)CTA_TILE) {
-                for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) emit.gather(b + j, (uint64_t)r, s[j]);
-            } else {
-                for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) keys[b + c0 + j] = s[j];
-            }
-            __syncthreads();
-        }
-        if (len <= (uint32_t)CTA_TILE) continue;
-        uint64_t *src = keys + b, *dst = scratch + b;
-        for (uint32_t w = CTA_TILE; w < len; w <<= 1) {
-            for (uint32_t lo = 0; lo < len; lo += 2 * w) {
-                const uint32_t na = len - lo < w ? len - lo : w;
-                const uint32_t rest = len - lo - na;
-                const uint32_t nb = rest < w ? rest : w;
-                merge_runs(src + lo, na, src + lo + na, nb, dst + lo);
-            }
-            __syncthreads();
-            uint64_t *t = src; src = dst; dst = t;
-        }
-        for (uint32_t j = threadIdx.x; j < len; j += blockDim.x) emit.gather(b + j, (uint64_t)r, src[j]);
         __syncthreads();
     }
 }
 
 template <class Emit>
-int launch_cta(cudaStream_t s, int64_t major_n, const uint32_t *start, uint64_t *keys, uint64_t *scratch,
-               const uint32_t *list, const uint32_t *counters, const Emit &emit) {
-    const size_t smem = (size_t)CTA_TILE * sizeof(uint64_t);
-    int rc = check_cuda(cudaFuncSetAttribute(cta_kernel<Emit>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                        "bucket: cta_kernel shared memory");
-    if (rc) return rc;
-    cta_kernel<Emit><<<152, CTA_THREADS, smem, s>>>(major_n, start, keys, scratch, list, counters, emit);
-    return check_cuda(cudaGetLastError(), "bucket cta_kernel");
+__global__ void __launch_bounds__(LONG_THREADS)
+long_merge_kernel(const uint32_t *__restrict__ start, const uint64_t *__restrict__ keys, LongRows longs, Emit emit) {
+    __shared__ uint64_t s[LONG_CHUNK];
+    constexpr int PER = LONG_CHUNK / LONG_THREADS;
+    const uint32_t nitems = longs.counters[1];
+    for (uint32_t q = blockIdx.x; q < nitems; q += gridDim.x) {
+        const uint2 item = longs.items[q];
+        const uint32_t b = start[item.x], len = start[item.x + 1] - b, c0 = item.y * LONG_CHUNK;
+        if (len <= (uint32_t)LONG_CHUNK) continue;  // the whole CTA
+        const uint32_t n = len - c0 < (uint32_t)LONG_CHUNK ? len - c0 : (uint32_t)LONG_CHUNK;
+        uint64_t k[PER];
+        uint32_t rank[PER];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const uint32_t j = (uint32_t)(u * LONG_THREADS) + threadIdx.x;
+            k[u] = j < n ? keys[b + c0 + j] : 0ull;
+            rank[u] = j;
+        }
+        const uint32_t nchunks = (len - 1) / LONG_CHUNK + 1;
+        for (uint32_t d = 0; d < nchunks; ++d) {
+            if (d == item.y) continue;
+            const uint32_t d0 = d * LONG_CHUNK;
+            const uint32_t m = len - d0 < (uint32_t)LONG_CHUNK ? len - d0 : (uint32_t)LONG_CHUNK;
+            for (uint32_t j = threadIdx.x; j < m; j += LONG_THREADS) s[j] = keys[b + d0 + j];
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                uint32_t lo = 0, hi = m;
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (s[mid] < k[u]) lo = mid + 1;
+                    else hi = mid;
+                }
+                rank[u] += lo;
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+            if ((uint32_t)(u * LONG_THREADS) + threadIdx.x < n) emit.gather(b + rank[u], (uint64_t)item.x, k[u]);
+    }
+}
+
+// The rows that the passes before left, keys in row order in `keys` (and values in `vals`).
+template <class VT, class Emit>
+int launch_long_rows(cudaStream_t s, const uint32_t *start, uint64_t *keys, const VT *vals, const LongRows &longs,
+                     const Emit &emit) {
+    warp_kernel<VT, Emit><<<152 * 8, WARP_CTA_THREADS, 0, s>>>(start, keys, vals, longs, emit);
+    long_sort_kernel<Emit><<<152 * 4, LONG_THREADS, 0, s>>>(start, keys, longs, emit);
+    long_merge_kernel<Emit><<<152 * 4, LONG_THREADS, 0, s>>>(start, keys, longs, emit);
+    return check_cuda(cudaGetLastError(), "bucket sort kernels");
 }
 
 inline unsigned grid_for(int64_t n, int64_t per_cta, int64_t cap) {
@@ -993,11 +1007,11 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
     const Layout L = layout(major_n, minor_n, nnz, VS, sc_tile);
     char *w = (char *)ws;
     uint32_t *cnt = (uint32_t *)(w + L.cnt), *start = (uint32_t *)(w + L.start);
-    uint32_t *bsums = (uint32_t *)(w + L.bsums), *list = (uint32_t *)(w + L.list);
-    uint32_t *counters = (uint32_t *)(w + L.counters);
+    uint32_t *bsums = (uint32_t *)(w + L.bsums);
+    const LongRows longs{(uint32_t *)(w + L.list), (uint2 *)(w + L.items), (uint32_t *)(w + L.counters)};
     uint64_t *key1 = (uint64_t *)(w + L.key1), *key2 = (uint64_t *)(w + L.key2);
     int rc = check_cuda(cudaMemsetAsync(cnt, 0, (size_t)L.ncnt * sizeof(uint32_t), s), "bucket: clear");
-    if (!rc) rc = check_cuda(cudaMemsetAsync(counters, 0, 4 * sizeof(uint32_t), s), "bucket: clear");
+    if (!rc) rc = check_cuda(cudaMemsetAsync(longs.counters, 0, 4 * sizeof(uint32_t), s), "bucket: clear");
     if (rc) return rc;
     const int64_t cap = 152 * 16;
     if (L.co.ok) {
@@ -1046,11 +1060,8 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
                             "bucket: fine_stage_kernel shared memory");
             if (rc) return rc;
             fine_stage_kernel<VT, Emit><<<(unsigned)(co.nb < sms ? co.nb : sms), ST_THREADS, sm, s>>>(
-                major_n, co, fcap, cstart, rec1, key2, val2, start, list, counters, emit);
-            warp_kernel<VT, Emit><<<152 * 8, WARP_CTA_THREADS, 0, s>>>(start, key2, val2, list, counters, emit);
-            rc = launch_cta(s, major_n, start, key2, key1, list, counters, emit);
-            if (rc) return rc;
-            return check_cuda(cudaGetLastError(), "bucket sort kernels");
+                major_n, co, fcap, cstart, rec1, key2, val2, start, longs, emit);
+            return launch_long_rows<VT, Emit>(s, start, key2, val2, longs, emit);
         }
         const size_t smem = fine_smem_bytes<VT>(co.cs);
         rc = check_cuda(cudaFuncSetAttribute(fine_kernel<VT, Emit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1058,11 +1069,8 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
                         "bucket: fine_kernel shared memory");
         if (rc) return rc;
         fine_kernel<VT, Emit><<<grid_for(co.nb, 1, 152 * 2), PC_THREADS, smem, s>>>(
-            major_n, co, cstart, rec1, key2, val2, start, list, counters, emit);
-        warp_kernel<VT, Emit><<<152 * 8, WARP_CTA_THREADS, 0, s>>>(start, key2, val2, list, counters, emit);
-        rc = launch_cta(s, major_n, start, key2, key1, list, counters, emit);
-        if (rc) return rc;
-        return check_cuda(cudaGetLastError(), "bucket sort kernels");
+            major_n, co, cstart, rec1, key2, val2, start, longs, emit);
+        return launch_long_rows<VT, Emit>(s, start, key2, val2, longs, emit);
     }
     if (nnz > 0) count_kernel<Src><<<grid_for(nnz, 256, cap), 256, 0, s>>>(src, nnz, major_n, cnt);
     rc = check_cuda(cudaGetLastError(), "bucket count_kernel");
@@ -1070,12 +1078,8 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
     if (!rc) rc = check_cuda(cudaMemsetAsync(cnt, 0, (size_t)L.ncnt * sizeof(uint32_t), s), "bucket: clear");
     if (rc) return rc;
     if (nnz > 0) place_kernel<Src><<<grid_for(nnz, 256, cap), 256, 0, s>>>(src, nnz, major_n, start, cnt, key1);
-    small_kernel<Emit><<<grid_for(major_n + 1, 256, 152 * 32), 256, 0, s>>>(major_n, start, key1, list, counters,
-                                                                             emit);
-    warp_kernel<NoValue, Emit><<<152 * 8, WARP_CTA_THREADS, 0, s>>>(start, key1, nullptr, list, counters, emit);
-    rc = launch_cta(s, major_n, start, key1, key2, list, counters, emit);
-    if (rc) return rc;
-    return check_cuda(cudaGetLastError(), "bucket sort kernels");
+    small_kernel<Emit><<<grid_for(major_n + 1, 256, 152 * 32), 256, 0, s>>>(major_n, start, key1, longs, emit);
+    return launch_long_rows<NoValue, Emit>(s, start, key1, nullptr, longs, emit);
 }
 
 }  // namespace bucket
