@@ -29,8 +29,11 @@
 // Matrices with more than 8191 x 4096 rows take the one-level form (count, place, and
 // small_kernel per row), whose stores are random.
 //
-// A source gives, for entry i, its 0-based major index (`major(i)`) and both indices
-// (`get(i, major, minor)`); an emitter receives each row's first position (`pointer(r,
+// A source is one or more parts, each a plain stretch of entries: src.parts(f) calls f(part, count,
+// first) with the position of the part's first entry.  A part gives, for its entry i, the 0-based
+// major index (`major(i)`), both indices (`get(i, major, minor)`) and, where values are carried,
+// `value(i)`.  (One source for all parts, asking for every entry which part it is in, kept the loads
+// from being issued together: counting 42M entries 155 us against 87.) an emitter receives each row's first position (`pointer(r,
 // first)`, r = 0..major_n) and every entry's sorted position with its row, key and value
 // (`put(p, r, key, value)`, or `gather(p, r, key)` where the value is not carried).
 //
@@ -55,15 +58,16 @@ constexpr int ROWS_MAX = 4096;     // rows per coarse bucket
 constexpr int COARSE_MAX = 8192;   // coarse buckets, the invalid-row bucket included
 constexpr int PB_THREADS = 256, PB_ITEMS = 8;
 constexpr int PC_THREADS = 512;
-constexpr int STAGE_BYTES = 96 * 1024;  // fine_kernel's shared staging of one coarse bucket
+constexpr int STAGE_BYTES = 96 * 1024;  // a bucket of average rows fills at most half of this (coarse_plan)
 
-struct NoValue {};  // the COO sums carry no values (they sum by input position)
+struct NoValue {};  // no values carried: the COO sums, which gather them by input position
 
 template <class VT> __host__ __device__ constexpr size_t carried_size() {
     return std::is_same<VT, NoValue>::value ? 0 : sizeof(VT);
 }
-// Entries of a coarse bucket that fine_kernel stages in shared memory (key + value each).
-template <class VT> __host__ __device__ constexpr int stage_entries() { return (int)(STAGE_BYTES / (8 + carried_size<VT>())); }
+// Entries of a coarse bucket that fine_kernel stages in shared memory, a key each and with values
+// the number of its record: 105 KB, so that two CTAs fit an SM beside the offsets of 1024 rows.
+template <class VT> __host__ __device__ constexpr int stage_entries() { return carried_size<VT>() ? 10496 : 12288; }
 
 struct Coarse {
     bool ok;
@@ -291,7 +295,7 @@ coarse_count_kernel(Src src, int64_t nnz, int64_t major_n, int cs, int64_t nb, u
 #endif
 template <class Src, class VT>
 __global__ void __launch_bounds__(PB_THREADS, GSA_PB_MIN_BLOCKS)
-coarse_place_kernel(Src src, const VT *__restrict__ vals_in, int64_t nnz, int64_t major_n, Coarse co,
+coarse_place_kernel(Src src, int64_t nnz, int64_t first, int64_t major_n, Coarse co,
                     uint32_t *__restrict__ cfill, Rec<VT> *__restrict__ rec1) {
     const int cs = co.cs;
     const int64_t nb = co.nb;
@@ -317,7 +321,7 @@ coarse_place_kernel(Src src, const VT *__restrict__ vals_in, int64_t nnz, int64_
             mns[q] = 0;
             if (e < nnz) {
                 src.get(e, mjs[q], mns[q]);
-                if constexpr (HAS_VAL) val[q] = vals_in[e];
+                if constexpr (HAS_VAL) val[q] = src.value(e);
             }
         }
 #pragma unroll
@@ -329,7 +333,7 @@ coarse_place_kernel(Src src, const VT *__restrict__ vals_in, int64_t nnz, int64_
             const uint64_t lrow = in ? (uint64_t)(mj - ((int64_t)d << cs)) : 0;
             // the minor index masked to its field, so that an index outside the matrix cannot
             // reach the row bits
-            key[q] = shl64(lrow, co.mb + co.pb) | ((((uint64_t)mn) & low_mask(co.mb)) << co.pb) | (uint64_t)e;
+            key[q] = shl64(lrow, co.mb + co.pb) | ((((uint64_t)mn) & low_mask(co.mb)) << co.pb) | (uint64_t)(first + e);
             packed[q] = e < nnz ? (d << 16) | atomicAdd(&s_run[d], 1u) : 0u;
         }
         __syncthreads();
@@ -816,13 +820,13 @@ __global__ void count_kernel(Src src, int64_t nnz, int64_t major_n, uint32_t *__
 }
 
 template <class Src>
-__global__ void place_kernel(Src src, int64_t nnz, int64_t major_n, const uint32_t *__restrict__ start,
+__global__ void place_kernel(Src src, int64_t nnz, int64_t first, int64_t major_n, const uint32_t *__restrict__ start,
                              uint32_t *__restrict__ fill, uint64_t *__restrict__ keys) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
         int64_t mj, mn;
         src.get(i, mj, mn);
         const int64_t r = (uint64_t)mj < (uint64_t)major_n ? mj : major_n;
-        keys[(uint64_t)start[r] + atomicAdd(&fill[r], 1u)] = ((uint64_t)(uint32_t)mn << 32) | (uint32_t)i;
+        keys[(uint64_t)start[r] + atomicAdd(&fill[r], 1u)] = ((uint64_t)(uint32_t)mn << 32) | (uint32_t)(first + i);
     }
 }
 
@@ -997,11 +1001,11 @@ inline unsigned grid_for(int64_t n, int64_t per_cta, int64_t cap) {
     return (unsigned)(b > 0 ? b : 1);
 }
 
-// The whole sort.  vals_in: the values to carry (VT = NoValue: none).  scan(s, in, out, n,
-// bsums) is the library's exclusive scan of uint32.
-template <class Src, class VT, class Emit, class Scan>
-int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Src &src, const VT *vals_in,
-         const Emit &emit, void *ws, Scan scan, size_t sc_tile) {
+// The whole sort.  VT: the type of the values to carry, which the parts give (NoValue: none).
+// scan(s, in, out, n, bsums) is the library's exclusive scan of uint32.
+template <class VT, class Src, class Emit, class Scan>
+int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Src &src, const Emit &emit, void *ws,
+         Scan scan, size_t sc_tile) {
     constexpr size_t VS = std::is_same<VT, NoValue>::value ? 0 : sizeof(VT);
     static_assert(sizeof(Rec<VT>) == rec_size(VS), "record size of the layout");
     const Layout L = layout(major_n, minor_n, nnz, VS, sc_tile);
@@ -1033,9 +1037,12 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
         // dynamic shared memory the staged kernels may take (their static arrays stay below 512 B)
         const size_t smax = optin > 1024 ? (size_t)optin - 512 : 0;
         // the counting pass: six CTAs of 32 KB histograms per SM, each flushing its counts once
-        if (nnz > 0)
-            coarse_count_kernel<Src><<<grid_for(nnz, PB_THREADS * PB_ITEMS, staged ? (int64_t)sms * 6 : cap),
-                                       PB_THREADS, 0, s>>>(src, nnz, major_n, co.cs, co.nb, cnt);
+        src.parts([&](const auto &part, int64_t n, int64_t) {
+            using P = std::decay_t<decltype(part)>;
+            if (n > 0)
+                coarse_count_kernel<P><<<grid_for(n, PB_THREADS * PB_ITEMS, staged ? (int64_t)sms * 6 : cap),
+                                         PB_THREADS, 0, s>>>(part, n, major_n, co.cs, co.nb, cnt);
+        });
         rc = check_cuda(cudaGetLastError(), "bucket coarse_count_kernel");
         if (!rc) rc = scan(s, cnt, cstart, co.nb + 1, bsums);  // cstart[nb] = nnz
         // the fill cursors start at the buckets' first slots
@@ -1044,9 +1051,12 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
                                             cudaMemcpyDeviceToDevice, s),
                             "bucket: cursors");
         if (rc) return rc;
-        if (nnz > 0)
-            coarse_place_kernel<Src, VT><<<grid_for(nnz, PB_THREADS * PB_ITEMS, cap), PB_THREADS, 0, s>>>(
-                src, vals_in, nnz, major_n, co, cnt, rec1);
+        src.parts([&](const auto &part, int64_t n, int64_t first) {
+            using P = std::decay_t<decltype(part)>;
+            if (n > 0)
+                coarse_place_kernel<P, VT><<<grid_for(n, PB_THREADS * PB_ITEMS, cap), PB_THREADS, 0, s>>>(
+                    part, n, first, major_n, co, cnt, rec1);
+        });
         // the staged pass C copies whole 16-byte-aligned records (conversions carry values); it
         // pays where rows are short (thread-sorted): with longer rows, most entries are sorted by
         // warps, whose uneven work two CTAs per SM overlap better (power-law rows averaging 16
@@ -1072,12 +1082,18 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
             major_n, co, cstart, rec1, key2, val2, start, longs, emit);
         return launch_long_rows<VT, Emit>(s, start, key2, val2, longs, emit);
     }
-    if (nnz > 0) count_kernel<Src><<<grid_for(nnz, 256, cap), 256, 0, s>>>(src, nnz, major_n, cnt);
+    src.parts([&](const auto &part, int64_t n, int64_t) {
+        using P = std::decay_t<decltype(part)>;
+        if (n > 0) count_kernel<P><<<grid_for(n, 256, cap), 256, 0, s>>>(part, n, major_n, cnt);
+    });
     rc = check_cuda(cudaGetLastError(), "bucket count_kernel");
     if (!rc) rc = scan(s, cnt, start, major_n + 2, bsums);
     if (!rc) rc = check_cuda(cudaMemsetAsync(cnt, 0, (size_t)L.ncnt * sizeof(uint32_t), s), "bucket: clear");
     if (rc) return rc;
-    if (nnz > 0) place_kernel<Src><<<grid_for(nnz, 256, cap), 256, 0, s>>>(src, nnz, major_n, start, cnt, key1);
+    src.parts([&](const auto &part, int64_t n, int64_t first) {
+        using P = std::decay_t<decltype(part)>;
+        if (n > 0) place_kernel<P><<<grid_for(n, 256, cap), 256, 0, s>>>(part, n, first, major_n, start, cnt, key1);
+    });
     small_kernel<Emit><<<grid_for(major_n + 1, 256, 152 * 32), 256, 0, s>>>(major_n, start, key1, longs, emit);
     return launch_long_rows<NoValue, Emit>(s, start, key1, nullptr, longs, emit);
 }

@@ -380,10 +380,14 @@ size_t coo_to_compressed_workspace_size(int64_t m, int64_t n, int64_t nnz, bool 
     return sort_layout(nnz).bytes;
 }
 
-template <typename I>
+template <typename V, typename I>
 struct PairSource {
     const I *mj, *mn;
+    const V *val;
     int base;
+    int64_t nnz;
+    template <typename F> void parts(F &&f) const { f(*this, nnz, (int64_t)0); }
+    __device__ __forceinline__ V value(int64_t i) const { return val[i]; }
     __device__ __forceinline__ int64_t major(int64_t i) const { return (int64_t)__ldg(mj + i) - base; }
     __device__ __forceinline__ void get(int64_t i, int64_t &a, int64_t &b) const {
         a = (int64_t)__ldg(mj + i) - base;
@@ -439,10 +443,10 @@ int launch_coo_to_compressed(cudaStream_t s, bool colmajor, int64_t m, int64_t n
     if (bucket_fits(major_n, minor_n, nnz)) {
         if (ws_bytes < bucket::layout(major_n, minor_n, nnz, sizeof(V), SC_TILE).bytes)
             return fail(GSA_ERR_INVALID_ARG, "conversion workspace too small");
-        PairSource<I> src{major, minor, base};
+        const PairSource<V, I> src{major, minor, val, base, nnz};
         CompressedEmit<V, I> emit{ptr_out, idx_out, val_out, val, base, major_n, nnz};
         timer_before(s);
-        int rc = bucket::sort(s, major_n, minor_n, nnz, src, val, emit, ws, exclusive_scan_u32, SC_TILE);
+        int rc = bucket::sort<V>(s, major_n, minor_n, nnz, src, emit, ws, exclusive_scan_u32, SC_TILE);
         timer_after(s);
         return rc;
     }
@@ -728,63 +732,136 @@ __device__ __forceinline__ V sum_source_value(const SumSources &src, uint32_t p,
     return negate_if(conj_if(v, src.conj[w] != 0), src.neg[w] != 0);
 }
 
-// flags[i] = 1 where sorted entry i starts a run whose sum is nonzero; the sum goes to sums[i].
-template <typename V>
-__global__ void run_sum_kernel(SumSources src, int64_t total, const uint64_t *__restrict__ keys,
-                               const uint32_t *__restrict__ perm, V lambda, V *__restrict__ sums,
-                               uint32_t *__restrict__ flags) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= total; i += (int64_t)gridDim.x * blockDim.x) {
-        uint32_t f = 0;
-        if (i < total) {
-            const uint64_t k = keys[i];
-            if (i == 0 || keys[i - 1] != k) {
-                V acc = sum_source_value<V>(src, perm[i], lambda);
-                for (int64_t j = i + 1; j < total && keys[j] == k; ++j)
-                    acc = add(acc, sum_source_value<V>(src, perm[j], lambda));
-                sums[i] = acc;
-                f = is_zero(acc) ? 0u : 1u;
-            }
+constexpr int RUN_THREADS = 256, RUN_ITEMS = 8;
+constexpr int RUN_WARPS = RUN_THREADS / 32;
+constexpr int RUN_TILE = RUN_THREADS * RUN_ITEMS;
+static_assert(RUN_ITEMS * RUN_WARPS == 64, "run_places scans two counts per lane");
+
+// s_at[64]: entries kept of each 32 consecutive ones of a tile -> places before them; the CTA's
+// total is returned.  All threads call this between barriers of their own.
+__device__ __forceinline__ void run_places(uint32_t *s_at, uint32_t *s_total) {
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        const uint32_t a = s_at[2 * lane], b = s_at[2 * lane + 1];
+        uint32_t x = a + b;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += y;
         }
-        flags[i] = f;
+        s_at[2 * lane] = x - a - b;
+        s_at[2 * lane + 1] = x - b;
+        if (lane == 31) *s_total = x;
     }
 }
 
+// A CTA per tile of 2048 sorted entries.  The values of all of them are gathered at once (eight
+// independent reads per thread) into shared memory; then each run of equal keys is summed where it
+// starts, left to right (past the tile's end from global memory), and the nonzero sums are left at
+// the tile's first positions of skeys and sums, in order, their number in counts.  Bound by the
+// gathers from values larger than L2, a sector and its DRAM burst each: 42M Float64 entries 610 us.
+// (One flag and one sum per entry, and a scan of the flags, took 590 and 215 us, and the writing of
+// the result from them 215 against 120.  Carrying the values through the sort instead takes the
+// gathers out, run sums 210 us, and costs its passes 580.)
+template <typename V>
+__global__ void __launch_bounds__(RUN_THREADS)
+run_sum_kernel(SumSources src, int64_t total, const uint64_t *__restrict__ keys, const uint32_t *__restrict__ perm,
+               V lambda, uint64_t *__restrict__ skeys, V *__restrict__ sums, uint32_t *__restrict__ counts) {
+    __shared__ V s_val[RUN_TILE];
+    __shared__ uint64_t s_key[RUN_TILE + 1];  // s_key[i]: the key before entry i of the tile
+    __shared__ uint32_t s_at[64], s_total;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t t0 = (int64_t)blockIdx.x * RUN_TILE;
+    const int n = total - t0 < RUN_TILE ? (int)(total - t0) : RUN_TILE;
+    uint32_t p[RUN_ITEMS];
+#pragma unroll
+    for (int u = 0; u < RUN_ITEMS; ++u) {
+        const int i = u * RUN_THREADS + threadIdx.x;
+        p[u] = i < n ? perm[t0 + i] : 0u;
+        if (i < n) s_key[i + 1] = keys[t0 + i];
+    }
+    if (threadIdx.x == 0) s_key[0] = t0 > 0 ? keys[t0 - 1] : ~keys[0];
+    V v[RUN_ITEMS];
+#pragma unroll
+    for (int u = 0; u < RUN_ITEMS; ++u)
+        v[u] = u * RUN_THREADS + (int)threadIdx.x < n ? sum_source_value<V>(src, p[u], lambda) : VT<V>::zero();
+#pragma unroll
+    for (int u = 0; u < RUN_ITEMS; ++u) s_val[u * RUN_THREADS + threadIdx.x] = v[u];
+    __syncthreads();
+    unsigned kept[RUN_ITEMS];
+#pragma unroll
+    for (int u = 0; u < RUN_ITEMS; ++u) {
+        const int i = u * RUN_THREADS + threadIdx.x;
+        bool keep = false;
+        if (i < n && s_key[i] != s_key[i + 1]) {
+            const uint64_t k = s_key[i + 1];
+            int j = i + 1;
+            for (; j < n && s_key[j + 1] == k; ++j) v[u] = add(v[u], s_val[j]);
+            if (j == n)
+                for (int64_t g = t0 + n; g < total && keys[g] == k; ++g)
+                    v[u] = add(v[u], sum_source_value<V>(src, perm[g], lambda));
+            keep = !is_zero(v[u]);
+        }
+        kept[u] = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) s_at[u * RUN_WARPS + w] = (uint32_t)__popc(kept[u]);
+    }
+    __syncthreads();
+    run_places(s_at, &s_total);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < RUN_ITEMS; ++u) {
+        if (!((kept[u] >> lane) & 1u)) continue;
+        const int64_t at = t0 + s_at[u * RUN_WARPS + w] + __popc(kept[u] & ((1u << lane) - 1));
+        skeys[at] = s_key[u * RUN_THREADS + threadIdx.x + 1];
+        sums[at] = v[u];
+    }
+    if (threadIdx.x == 0) counts[blockIdx.x] = s_total;
+}
+
+// The tiles' sums to their places: tile b's are firsts[b] .. firsts[b + 1].
 template <typename V, typename I>
-__global__ void run_write_kernel(int64_t total, const uint64_t *__restrict__ keys, const uint32_t *__restrict__ pos,
-                                 const V *__restrict__ sums, int row_bits, int base, I *__restrict__ row_out,
-                                 I *__restrict__ col_out, V *__restrict__ val_out) {
+__global__ void __launch_bounds__(RUN_THREADS)
+run_write_kernel(const uint64_t *__restrict__ skeys, const V *__restrict__ sums, const uint32_t *__restrict__ firsts,
+                 int row_bits, int base, I *__restrict__ row_out, I *__restrict__ col_out, V *__restrict__ val_out) {
     const uint64_t mask = row_bits >= 64 ? ~0ull : ((1ull << row_bits) - 1);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t p = pos[i];
-        if (pos[i + 1] == p) continue;  // not a run start, or a zero sum
-        const uint64_t k = keys[i];
-        row_out[p] = (I)((int64_t)(k & mask) + base);
-        col_out[p] = (I)((int64_t)(row_bits >= 64 ? 0 : k >> row_bits) + base);
-        val_out[p] = sums[i];
+    const int64_t t0 = (int64_t)blockIdx.x * RUN_TILE;
+    const uint32_t f = firsts[blockIdx.x], n = firsts[blockIdx.x + 1] - f;
+#pragma unroll
+    for (int u = 0; u < RUN_ITEMS; ++u) {
+        const uint32_t i = (uint32_t)(u * RUN_THREADS) + threadIdx.x;
+        if (i >= n) break;
+        const uint64_t k = skeys[t0 + i];
+        row_out[f + i] = (I)((int64_t)(k & mask) + base);
+        col_out[f + i] = (I)((int64_t)(row_bits >= 64 ? 0 : k >> row_bits) + base);
+        val_out[f + i] = sums[t0 + i];
     }
 }
 
 // Column-major order: buckets are columns, the minor index is the row.
 template <typename I>
+struct SumPart {  // one COO source, its index arrays swapped where it is transposed
+    const I *col, *row;
+    int base;
+    __device__ __forceinline__ int64_t major(int64_t i) const { return (int64_t)__ldg(col + i) - base; }
+    __device__ __forceinline__ void get(int64_t i, int64_t &c, int64_t &r) const {
+        c = (int64_t)__ldg(col + i) - base;
+        r = (int64_t)__ldg(row + i) - base;
+    }
+};
+struct DiagPart {
+    __device__ __forceinline__ int64_t major(int64_t i) const { return i; }
+    __device__ __forceinline__ void get(int64_t i, int64_t &c, int64_t &r) const { c = r = i; }
+};
+template <typename I>
 struct SumSource {
     SumSources s;
     int base;
-    __device__ __forceinline__ void get(int64_t i, int64_t &col, int64_t &row) const {
-        if (i < s.nnz[0] + s.nnz[1]) {
-            const int w = i < s.nnz[0] ? 0 : 1;
-            const int64_t j = w ? i - s.nnz[0] : i;
-            const int64_t ri = (int64_t)__ldg((const I *)s.row[w] + j) - base;
-            const int64_t ci = (int64_t)__ldg((const I *)s.col[w] + j) - base;
-            row = s.trans[w] ? ci : ri;
-            col = s.trans[w] ? ri : ci;
-        } else {
-            row = col = i - s.nnz[0] - s.nnz[1];
+    template <typename F> void parts(F &&f) const {
+        for (int w = 0; w < 2; ++w) {
+            const I *row = (const I *)s.row[w], *col = (const I *)s.col[w];
+            f(s.trans[w] ? SumPart<I>{row, col, base} : SumPart<I>{col, row, base}, s.nnz[w], w ? s.nnz[0] : 0);
         }
-    }
-    __device__ __forceinline__ int64_t major(int64_t i) const {
-        int64_t c, r;
-        get(i, c, r);
-        return c;
+        f(DiagPart{}, s.n_diag, s.nnz[0] + s.nnz[1]);
     }
 };
 
@@ -802,7 +879,8 @@ struct KeyEmit {
 struct SumLayout {
     bool bucket;
     SortLayout sort;
-    size_t keys, perm, flags, pos, bsums, sums, bytes;
+    int64_t tiles;
+    size_t keys, perm, skeys, sums, firsts, bsums, bytes;
 };
 static SumLayout sum_layout(int64_t m, int64_t n, int64_t total, size_t vsize) {
     SumLayout L;
@@ -826,10 +904,11 @@ static SumLayout sum_layout(int64_t m, int64_t n, int64_t total, size_t vsize) {
         L.keys = passes % 2 ? kb : 0;
         L.perm = passes % 2 ? pb : pa;
     }
-    L.flags = cv.reserve<uint32_t>(total + 1);
-    L.pos = cv.reserve<uint32_t>(total + 1);
-    L.bsums = cv.reserve<uint32_t>(ceil_div(total + 1, SC_TILE) + 1);
+    L.tiles = ceil_div(total, RUN_TILE);
+    L.skeys = cv.reserve<uint64_t>(total);
     L.sums = cv.reserve<unsigned char>((size_t)total * vsize);
+    L.firsts = cv.reserve<uint32_t>(L.tiles + 1);
+    L.bsums = cv.reserve<uint32_t>(ceil_div(L.tiles + 1, SC_TILE) + 1);
     L.bytes = align_up(cv.off, 256);
     return L;
 }
@@ -857,15 +936,15 @@ int launch_coo_sum_count(cudaStream_t s, int64_t m, int64_t n, const SumSources 
     char *w = (char *)ws;
     uint64_t *keys = (uint64_t *)(w + L.keys);
     uint32_t *perm = (uint32_t *)(w + L.perm);
-    uint32_t *flags = (uint32_t *)(w + L.flags), *pos = (uint32_t *)(w + L.pos);
-    uint32_t *bs2 = (uint32_t *)(w + L.bsums);
+    uint32_t *firsts = (uint32_t *)(w + L.firsts), *bs2 = (uint32_t *)(w + L.bsums);
+    uint64_t *skeys = (uint64_t *)(w + L.skeys);
     V *sums = (V *)(w + L.sums);
+    const V lam = lambda ? *lambda : V{};
     int rc = GSA_OK;
     timer_before(s);
     if (L.bucket) {
-        SumSource<I> bs{src, base};
-        rc = bucket::sort(s, n, m, total, bs, (const bucket::NoValue *)nullptr, KeyEmit{keys, perm}, ws,
-                          exclusive_scan_u32, SC_TILE);
+        rc = bucket::sort<bucket::NoValue>(s, n, m, total, SumSource<I>{src, base}, KeyEmit{keys, perm}, ws,
+                                           exclusive_scan_u32, SC_TILE);
     } else {
         Carver cv(ws);
         uint64_t *ka = cv.take<uint64_t>(total), *kb = cv.take<uint64_t>(total);
@@ -891,14 +970,14 @@ int launch_coo_sum_count(cudaStream_t s, int64_t m, int64_t n, const SumSources 
         if (!rc && (ka != keys || pa != perm)) rc = fail(GSA_ERR_CUDA, "coo sum: sorted keys not where expected");
     }
     if (!rc) {
-        const V lam = lambda ? *lambda : V{};
-        run_sum_kernel<V><<<grid_for(total + 1, 256), 256, 0, s>>>(src, total, keys, perm, lam, sums, flags);
+        run_sum_kernel<V><<<(unsigned)L.tiles, RUN_THREADS, 0, s>>>(src, total, keys, perm, lam, skeys, sums, firsts);
         rc = check_cuda(cudaGetLastError(), "run_sum_kernel");
     }
-    if (!rc) rc = exclusive_scan_u32(s, flags, pos, total + 1, bs2);
+    if (!rc) rc = check_cuda(cudaMemsetAsync(firsts + L.tiles, 0, sizeof(uint32_t), s), "coo sum: clear");
+    if (!rc) rc = exclusive_scan_u32(s, firsts, firsts, L.tiles + 1, bs2);
     timer_after(s);
     uint32_t u = 0;
-    if (!rc) rc = check_cuda(cudaMemcpyAsync(&u, pos + total, sizeof(u), cudaMemcpyDeviceToHost, s), "coo sum: count");
+    if (!rc) rc = check_cuda(cudaMemcpyAsync(&u, firsts + L.tiles, sizeof(u), cudaMemcpyDeviceToHost, s), "coo sum: count");
     if (!rc) rc = check_cuda(cudaStreamSynchronize(s), "coo sum: sync");
     if (!rc) *kept = (int64_t)u;
     return rc;
@@ -910,12 +989,12 @@ int launch_coo_sum_copy(cudaStream_t s, int64_t m, int64_t n, int64_t total, int
     if (total <= 0) return GSA_OK;
     const SumLayout L = sum_layout(m, n, total, sizeof(V));
     const char *w = (const char *)ws;
-    const uint64_t *keys = (const uint64_t *)(w + L.keys);
-    const uint32_t *pos = (const uint32_t *)(w + L.pos);
+    const uint64_t *skeys = (const uint64_t *)(w + L.skeys);
+    const uint32_t *firsts = (const uint32_t *)(w + L.firsts);
     const V *sums = (const V *)(w + L.sums);
     timer_before(s);
-    run_write_kernel<V, I><<<grid_for(total, 256), 256, 0, s>>>(total, keys, pos, sums, L.bucket ? 32 : bits_for(m),
-                                                               base, row_out, col_out, val_out);
+    run_write_kernel<V, I><<<(unsigned)L.tiles, RUN_THREADS, 0, s>>>(skeys, sums, firsts, L.bucket ? 32 : bits_for(m),
+                                                                     base, row_out, col_out, val_out);
     timer_after(s);
     return check_cuda(cudaGetLastError(), "run_write_kernel");
 }
