@@ -94,6 +94,46 @@ cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s) {
     return cudaMallocAsync(p, bytes, s);
 }
 
+// A stream per device that only memory is given back on, ordered after an event of its last use.
+static std::atomic<cudaStream_t> g_free_streams[POOL_DEVICES];
+
+int scratch_free_after(int device, cudaEvent_t used, std::initializer_list<void *> mem) {
+    bool any = false;
+    for (void *p : mem) any = any || p;
+    if (!any) return GSA_OK;
+    int dev = 0;
+    const bool moved = cudaGetDevice(&dev) == cudaSuccess && dev != device;
+    if (moved) cudaSetDevice(device);
+    cudaStream_t fs = nullptr;
+    if (used && device >= 0 && device < POOL_DEVICES) {
+        fs = g_free_streams[device].load(std::memory_order_acquire);
+        if (!fs) {
+            std::lock_guard<std::mutex> hold(g_pools_lock);
+            fs = g_free_streams[device].load(std::memory_order_relaxed);
+            if (!fs) {
+                if (cudaStreamCreateWithFlags(&fs, cudaStreamNonBlocking) != cudaSuccess) {
+                    cudaGetLastError();
+                    fs = nullptr;
+                }
+                g_free_streams[device].store(fs, std::memory_order_release);
+            }
+        }
+    }
+    if (fs && cudaStreamWaitEvent(fs, used, 0) != cudaSuccess) {
+        cudaGetLastError();
+        fs = nullptr;
+    }
+    int rc = GSA_OK;
+    if (!fs) rc = check_cuda(cudaDeviceSynchronize(), "free: sync");
+    for (void *p : mem) {
+        if (!p) continue;
+        const int rc2 = check_cuda(fs ? cudaFreeAsync(p, fs) : cudaFree(p), "free");
+        if (!rc) rc = rc2;
+    }
+    if (moved) cudaSetDevice(dev);
+    return rc;
+}
+
 // Frees a plan's device memory.  Work on any stream may still read it, so the plan's device is
 // synchronized first (as cudaFree of a cudaMalloc allocation does by itself).
 static int plan_release(Plan *p) {

@@ -8,6 +8,7 @@
 #include <stddef.h>
 #include <math.h>
 
+#include <initializer_list>
 #include <type_traits>
 
 #include "../../include/gsa.h"
@@ -377,6 +378,9 @@ int radix_bits_for(int64_t count);  // bits that values 0 .. count - 1 need
 // back with cudaFreeAsync on a stream that is ordered after its last use, or with cudaFree once
 // the device has been synchronized (cudaFree waits for nothing on such memory).
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s);
+// Gives memory of scratch_alloc back once `used` has passed, without waiting for it here (NULL:
+// the device is synchronized instead).
+int scratch_free_after(int device, cudaEvent_t used, std::initializer_list<void *> mem);
 
 // Scratch of one call: the caller's buffer, or a stream-ordered allocation freed on the
 // same stream when the call returns.

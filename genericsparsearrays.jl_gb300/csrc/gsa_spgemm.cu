@@ -8,10 +8,14 @@
 // order, zero sums included.  That is m * n workspace.  Here each output row's products are
 // expanded in the same order and summed per column in that order -- so every entry gets the
 // reference's bits -- without a dense accumulator:
-//   1. entry_flops_kernel: products of every stored entry of P (the length of the Q row it
-//      selects); one scan; row_flops_kernel: products per output row from the scan at the row
-//      pointers, rows listed as tiny, small or big.
-//   2. tiny rows (at most 32 products), a thread each (tiny_kernel), and small rows (at most
+//   1. count_rows_kernel: a lane per row counts its products (the lengths of the Q rows it
+//      selects; a row of many entries by its whole warp), and counts the entries of rows of at most
+//      8 entries and 32 products at once by merging their Q rows, which sorted rows allow: the
+//      smallest next column, its products in order, the next.  merge_rows_kernel walks the same
+//      merges again for the values and writes 32 neighbouring rows together.  The other rows are
+//      listed as tiny, small or big.
+//   2. listed tiny rows (at most 32 products, unsorted or of more than 8 entries), a thread each
+//      (tiny_kernel), and small rows (at most
 //      256), a warp each (small_kernel): the row's products (column, value) expanded into
 //      shared memory in order; a product is the first of its column when no earlier one has
 //      the column; the count of first products is the row's entry count (symbolic pass); its
@@ -25,9 +29,10 @@
 // P and Q: CSR C = A * B runs over A's rows (P = A, Q = B); CSC C = A * B over B's columns
 // (P = B, Q = A).  Products are A-value times B-value with Julia's arithmetic (separate
 // multiply and add, textbook complex product), so the sums are the reference's bit for bit.
+#include <string>
 #include <type_traits>
 
-#include "gsa_internal.cuh"
+#include "gsa_rows.cuh"
 
 struct gsa_spgemm {
     int dtype = 0, itype = 0, csr = 1, base = 1;
@@ -39,7 +44,9 @@ struct gsa_spgemm {
     uint64_t pbig = 0;          // products of the big rows
     void *mem = nullptr;        // per-row arrays
     void *big = nullptr;        // big-row expansion and sort
-    size_t cnt_off = 0, cptr_off = 0, tiny_off = 0, small_off = 0, big_off = 0, counters_off = 0;
+    int device = 0;             // of both
+    cudaEvent_t used = nullptr; // after the handle's last work
+    size_t cptr_off = 0, tiny_off = 0, small_off = 0, big_off = 0, counters_off = 0, merged_off = 0;
     size_t boff_off = 0, keys_off = 0, flags_off = 0, rpos_off = 0, sums_off = 0;
     int cb = 0;                 // column bits of the big-row sort keys
 };
@@ -49,7 +56,8 @@ namespace {
 
 constexpr int SG_TINY_P = 32;     // products a thread sums in shared memory
 constexpr int SG_TINY_WARPS = 2;
-constexpr int SG_TINY_A = 8;      // A entries of a tiny row whose loads are issued together
+constexpr int SG_TINY_A = 8;      // entries of a merged row (their loads are issued together)
+constexpr int SG_MERGE_OUT = 16;  // entries of a merged row that are written together with its neighbours'
 constexpr int SG_WARP_P = 256;    // products a warp sums in shared memory
 constexpr int SG_THREADS = 128;   // 4 warps
 constexpr int SG_WARPS = SG_THREADS / 32;
@@ -78,64 +86,135 @@ __device__ __forceinline__ uint32_t lane_lt() {
     return lt;
 }
 
-// L[t] = products of P's stored entry t (the length of the Q outer entry it selects; 0 for an
-// index outside Q), t < nnz_p; L[nnz_p] = 0.
-// totals[0] += all products.
+// What count_rows_kernel finds besides the rows' counts: totals[0] all products, [1] the big rows';
+// counters[0] small rows, [1] big rows, [2] tiny rows.
+struct RowTotals {
+    unsigned long long totals[2];
+    uint32_t counters[4];
+};
+
+// The Q rows that up to SG_TINY_A entries of a row select, as cursors: entry c's row is at
+// cur[c], len[c] entries (0: none).  Returns the products.
 template <typename I>
-__global__ void entry_flops_kernel(int64_t nnz_p, const I *__restrict__ pi, const I *__restrict__ qp, int64_t q_outer,
-                                   int base, uint32_t *__restrict__ L, unsigned long long *__restrict__ totals) {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    unsigned long long sum = 0;  // one reduction and atomic per warp at the end
-#pragma unroll 4
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t <= nnz_p; t += stride) {
-        uint32_t len = 0;
-        if (t < nnz_p) {
-            const int64_t k = (int64_t)__ldg(pi + t) - base;
-            if ((uint64_t)k < (uint64_t)q_outer) len = (uint32_t)((int64_t)__ldg(qp + k + 1) - __ldg(qp + k));
-        }
-        L[t] = len;
-        sum += len;
-    }
+__device__ __forceinline__ uint64_t open_rows(const I *__restrict__ pi, const I *__restrict__ qp, int64_t q_outer, int base,
+                                              int64_t b, int n, Off<I> (&cur)[SG_TINY_A], uint32_t (&len)[SG_TINY_A]) {
+    int64_t k[SG_TINY_A];
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&totals[0], sum);
+    for (int c = 0; c < SG_TINY_A; ++c) k[c] = c < n ? (int64_t)__ldg(pi + b + c) - base : -1;
+    uint64_t f = 0;
+#pragma unroll
+    for (int c = 0; c < SG_TINY_A; ++c) {
+        const bool ok = (uint64_t)k[c] < (uint64_t)q_outer;
+        const int64_t q0 = ok ? (int64_t)__ldg(qp + k[c]) - base : 0;
+        len[c] = ok ? (uint32_t)((int64_t)__ldg(qp + k[c] + 1) - base - q0) : 0u;
+        cur[c] = (Off<I>)q0;
+        f += len[c];
+    }
+    return f;
 }
 
-// Products per outer entry of P from the scanned entry counts (the host has checked that all
-// products together number fewer than 2^32, so the scan does not wrap); rows listed small or
-// big; counters: [2] tiny rows (at most 32 products), [0] small rows (at most 256), [1] big
-// rows; totals[1]: big-row products.
-template <typename I>
-__global__ void row_flops_kernel(int64_t outer_n, const I *__restrict__ pp, int base, const uint32_t *__restrict__ S,
-                                 uint32_t *__restrict__ cnt, uint32_t *__restrict__ tiny_list,
-                                 uint32_t *__restrict__ small_list, uint32_t *__restrict__ big_list,
-                                 uint32_t *__restrict__ counters, unsigned long long *__restrict__ totals) {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t o0 = (int64_t)blockIdx.x * blockDim.x; o0 < outer_n; o0 += stride) {
-        const int64_t o = o0 + threadIdx.x;
-        const bool valid = o < outer_n;
-        uint32_t f = 0;
-        if (valid) {
-            const int64_t b = (int64_t)__ldg(pp + o) - base, e = (int64_t)__ldg(pp + o + 1) - base;
-            f = e > b ? S[e] - S[b] : 0u;
-            cnt[o] = 0;
-        }
-        const bool is_tiny = valid && f > 0 && f <= (uint32_t)SG_TINY_P;
-        const bool is_small = valid && f > (uint32_t)SG_TINY_P && f <= (uint32_t)SG_WARP_P;
-        const bool is_big = valid && f > (uint32_t)SG_WARP_P;
-        const unsigned ms = __ballot_sync(0xffffffffu, is_small), mb = __ballot_sync(0xffffffffu, is_big);
-        const unsigned mt = __ballot_sync(0xffffffffu, is_tiny);
-        const int lane = threadIdx.x & 31;
-        const unsigned lt = lane_lt();
-        unsigned long long fb = is_big ? f : 0;
+// Merges the open rows of a row of at most SG_TINY_P products: visit(j) for every column j in
+// increasing order after take(c, at) for each of its products in the reference's order (entries in
+// order, each Q row in order).  False, with part of them visited, when a Q row is not sorted.  (A
+// second column held per cursor, loaded one advance ahead, was slower: 591 us against 510 for
+// merge_rows_kernel on the 2048^2 grid, for its registers.)
+template <typename I, typename Take, typename Visit>
+__device__ __forceinline__ bool merge_open_rows(const I *__restrict__ qi, int base, Off<I> (&cur)[SG_TINY_A],
+                                                uint32_t (&len)[SG_TINY_A], Take &&take, Visit &&visit) {
+    constexpr uint32_t END = 0xffffffffu;
+    uint32_t jc[SG_TINY_A];
+    bool sorted = true;
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) fb += __shfl_xor_sync(0xffffffffu, fb, d);
+    for (int c = 0; c < SG_TINY_A; ++c) {
+        jc[c] = len[c] ? (uint32_t)((int64_t)__ldg(qi + cur[c]) - base) : END;
+        if (len[c] && jc[c] == END) sorted = false;  // a column that the end mark cannot stand beside
+    }
+    for (int guard = 0; sorted && guard <= SG_TINY_P; ++guard) {
+        uint32_t jmin = jc[0];
+#pragma unroll
+        for (int c = 1; c < SG_TINY_A; ++c) jmin = jc[c] < jmin ? jc[c] : jmin;
+        if (jmin == END) break;
+#pragma unroll
+        for (int c = 0; c < SG_TINY_A; ++c) {
+            while (jc[c] == jmin) {
+                take(c, cur[c]);
+                ++cur[c];
+                if (--len[c]) {
+                    jc[c] = (uint32_t)((int64_t)__ldg(qi + cur[c]) - base);
+                    if (jc[c] < jmin || jc[c] == END) {
+                        sorted = false;
+                        jc[c] = END;
+                    }
+                } else {
+                    jc[c] = END;
+                }
+            }
+        }
+        visit(jmin);
+    }
+    return sorted;
+}
+
+// A lane per row (of 32 neighbouring ones per warp): products, and for rows that merge_rows_kernel
+// takes (a bit in merged) their entries, into cnt; big rows leave their products there.  Bound by
+// the merges' instructions (issue slots 75 % busy).  The 2048^2 grid's
+// 105M products: 250 us; a flop count per stored entry, a scan of all of them, a pass over the rows
+// and tiny_kernel's symbolic pass took 665.
+template <typename I>
+__global__ void __launch_bounds__(SG_THREADS)
+count_rows_kernel(int64_t outer_n, const I *__restrict__ pp, const I *__restrict__ pi, const I *__restrict__ qp,
+                  const I *__restrict__ qi, int64_t q_outer, int base, uint32_t *__restrict__ cnt,
+                  uint32_t *__restrict__ merged, uint32_t *__restrict__ tiny_list, uint32_t *__restrict__ small_list,
+                  uint32_t *__restrict__ big_list, RowTotals *__restrict__ totals) {
+    __shared__ unsigned long long s_all, s_big;
+    if (threadIdx.x == 0) s_all = s_big = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    unsigned long long all = 0, allbig = 0;
+    const int64_t stride = (int64_t)gridDim.x * SG_THREADS;
+    for (int64_t row0 = (int64_t)blockIdx.x * SG_THREADS + (threadIdx.x & ~31); row0 < outer_n; row0 += stride) {
+        const int64_t o = row0 + lane;
+        const bool valid = o < outer_n;
+        int64_t b = 0, n = 0;
+        if (valid) {
+            b = (int64_t)__ldg(pp + o) - base;
+            n = (int64_t)__ldg(pp + o + 1) - base - b;
+        }
+        const bool few = n <= SG_TINY_A;
+        Off<I> cur[SG_TINY_A];
+        uint32_t len[SG_TINY_A];
+        uint64_t f = open_rows<I>(pi, qp, q_outer, base, b, few ? (int)(n > 0 ? n : 0) : 0, cur, len);
+        for (unsigned todo = __ballot_sync(0xffffffffu, !few); todo; todo &= todo - 1) {  // a row by its whole warp
+            const int l = __ffs(todo) - 1;
+            const int64_t bl = __shfl_sync(0xffffffffu, b, l), el = bl + __shfl_sync(0xffffffffu, n, l);
+            unsigned long long x = 0;
+#pragma unroll 4
+            for (int64_t t = bl + lane; t < el; t += 32) {
+                const int64_t k = (int64_t)__ldg(pi + t) - base;
+                if ((uint64_t)k < (uint64_t)q_outer) x += (uint32_t)((int64_t)__ldg(qp + k + 1) - __ldg(qp + k));
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+            if (lane == l) f = x;
+        }
+        uint32_t count = 0;
+        bool done = few && f > 0 && f <= (uint64_t)SG_TINY_P;
+        if (done) done = merge_open_rows<I>(qi, base, cur, len, [](int, Off<I>) {}, [&](uint32_t) { ++count; });
+        __syncwarp();
+        const bool is_tiny = !done && f > 0 && f <= (uint64_t)SG_TINY_P;
+        const bool is_small = f > (uint64_t)SG_TINY_P && f <= (uint64_t)SG_WARP_P, is_big = f > (uint64_t)SG_WARP_P;
+        if (valid) cnt[o] = done ? count : (is_big ? (uint32_t)f : 0u);
+        const unsigned md = __ballot_sync(0xffffffffu, done);
+        if (lane == 0) merged[row0 >> 5] = md;
+        all += f;
+        if (is_big) allbig += f;
+        const unsigned ms = __ballot_sync(0xffffffffu, is_small), mb = __ballot_sync(0xffffffffu, is_big);
+        const unsigned mt = __ballot_sync(0xffffffffu, is_tiny), lt = lane_lt();
         uint32_t bs = 0, bb = 0, bt = 0;
         if (lane == 0) {
-            if (mt) bt = atomicAdd(&counters[2], (uint32_t)__popc(mt));
-            if (ms) bs = atomicAdd(&counters[0], (uint32_t)__popc(ms));
-            if (mb) bb = atomicAdd(&counters[1], (uint32_t)__popc(mb));
-            if (fb) atomicAdd(&totals[1], fb);
+            if (ms) bs = atomicAdd(&totals->counters[0], (uint32_t)__popc(ms));
+            if (mb) bb = atomicAdd(&totals->counters[1], (uint32_t)__popc(mb));
+            if (mt) bt = atomicAdd(&totals->counters[2], (uint32_t)__popc(mt));
         }
         bs = __shfl_sync(0xffffffffu, bs, 0);
         bb = __shfl_sync(0xffffffffu, bb, 0);
@@ -144,8 +223,75 @@ __global__ void row_flops_kernel(int64_t outer_n, const I *__restrict__ pp, int 
         if (is_small) small_list[bs + __popc(ms & lt)] = (uint32_t)o;
         if (is_big) big_list[bb + __popc(mb & lt)] = (uint32_t)o;
     }
+    atomicAdd(&s_all, all);
+    if (allbig) atomicAdd(&s_big, allbig);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (s_all) atomicAdd(&totals->totals[0], s_all);
+        if (s_big) atomicAdd(&totals->totals[1], s_big);
+    }
 }
 
+// The entries of the merged rows, a lane per row, 32 neighbouring rows per warp: the warp's rows
+// leave their first SG_MERGE_OUT entries in shared memory and write them together, two rows at a
+// time, as one stretch of the result.  (A thread writing its own row sent every entry as a store
+// of its own, 109M of them for the 2048^2 grid: 940 us against 510.)
+template <typename V, typename I>
+__global__ void __launch_bounds__(SG_THREADS)
+merge_rows_kernel(int64_t outer_n, const uint32_t *__restrict__ merged, const I *__restrict__ pp,
+                  const I *__restrict__ pi, const V *__restrict__ pv, const I *__restrict__ qp,
+                  const I *__restrict__ qi, const V *__restrict__ qv, int64_t q_outer, int base, bool csr,
+                  const uint32_t *__restrict__ cptr, I *__restrict__ idx_out, V *__restrict__ val_out) {
+    constexpr int LD = 33;  // slot s of lane l at s * 33 + l: neither phase meets itself in a bank
+    __shared__ uint32_t s_j[SG_WARPS][SG_MERGE_OUT * LD];
+    __shared__ V s_v[SG_WARPS][SG_MERGE_OUT * LD];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t row0 = (int64_t)blockIdx.x * SG_THREADS + (threadIdx.x & ~31);
+    if (row0 >= outer_n) return;  // the whole warp
+    const unsigned md = __ldg(merged + (row0 >> 5));
+    if (!md) return;
+    const bool mine = (md >> lane) & 1u;
+    const int64_t o = row0 + lane;
+    uint32_t out0 = 0, count = 0;
+    if (mine) {
+        const int64_t b = (int64_t)__ldg(pp + o) - base;
+        const int n = (int)((int64_t)__ldg(pp + o + 1) - base - b);
+        out0 = cptr[o];
+        Off<I> cur[SG_TINY_A];
+        uint32_t len[SG_TINY_A];
+        V a[SG_TINY_A];
+#pragma unroll
+        for (int c = 0; c < SG_TINY_A; ++c) a[c] = c < n ? ldg(pv + b + c) : VT<V>::zero();
+        open_rows<I>(pi, qp, q_outer, base, b, n, cur, len);
+        V acc = VT<V>::zero();
+        merge_open_rows<I>(
+            qi, base, cur, len, [&](int c, Off<I> at) { acc = add(acc, product(a[c], ldg(qv + at), csr)); },
+            [&](uint32_t j) {
+                if (count < (uint32_t)SG_MERGE_OUT) {
+                    s_j[w][count * LD + lane] = j;
+                    s_v[w][count * LD + lane] = acc;
+                } else {
+                    idx_out[out0 + count] = (I)((int64_t)j + base);
+                    val_out[out0 + count] = acc;
+                }
+                ++count;
+                acc = VT<V>::zero();
+            });
+    }
+    __syncwarp();
+    const uint32_t together = count < (uint32_t)SG_MERGE_OUT ? count : (uint32_t)SG_MERGE_OUT;
+    const int t = lane & (SG_MERGE_OUT - 1);
+    static_assert(SG_MERGE_OUT == 16, "two rows per step of a warp");
+#pragma unroll 4
+    for (int l0 = 0; l0 < 32; l0 += 2) {
+        const int l = l0 + (lane >> 4);
+        const uint32_t nl = __shfl_sync(0xffffffffu, together, l), at = __shfl_sync(0xffffffffu, out0, l) + t;
+        if ((uint32_t)t < nl) {
+            idx_out[at] = (I)((int64_t)s_j[w][t * LD + l] + base);
+            val_out[at] = s_v[w][t * LD + l];
+        }
+    }
+}
 
 // Thread per listed tiny row (at most SG_TINY_P products): the same expansion, sums and
 // positions as small_kernel, each thread in its own column of the warp's shared block
@@ -386,18 +532,11 @@ small_kernel(const uint32_t *__restrict__ list, const uint32_t *__restrict__ cou
 
 // ---- big rows ----------------------------------------------------------------
 
-// flops of each big row, for the scan of their expansion offsets
-template <typename I>
-__global__ void big_flops_kernel(const uint32_t *__restrict__ list, uint32_t nbig, const I *__restrict__ pp, int base,
-                                 const uint32_t *__restrict__ S, uint32_t *__restrict__ bflops) {
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q <= nbig; q += gridDim.x * blockDim.x) {
-        uint32_t f = 0;
-        if (q < nbig) {
-            const uint32_t o = list[q];
-            f = S[(int64_t)__ldg(pp + o + 1) - base] - S[(int64_t)__ldg(pp + o) - base];
-        }
-        bflops[q] = f;
-    }
+// products of each big row (left in cnt), for the scan of their expansion offsets
+__global__ void big_flops_kernel(const uint32_t *__restrict__ list, uint32_t nbig, const uint32_t *__restrict__ cnt,
+                                 uint32_t *__restrict__ bflops) {
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q <= nbig; q += gridDim.x * blockDim.x)
+        bflops[q] = q < nbig ? cnt[list[q]] : 0u;
 }
 
 // CTA per big row: its products written from boff[q], in the reference's order, as key
@@ -526,24 +665,22 @@ unsigned sg_grid(int64_t n, int64_t per_cta, int64_t cap) {
     return (unsigned)(b > 0 ? b : 1);
 }
 
-// Per-row arrays of a product (one allocation): entry flops and their scan, row counts and
-// their scan, the two row lists, counters and totals, scan scratch.
+// Per-row arrays of a product (one allocation): row counts and their scan, the merged rows' bits,
+// the row lists, totals, scan scratch.
 struct RowLayout {
-    size_t L, cnt, cptr, tiny, small, big, counters, totals, bsums, bytes;
+    size_t cnt, cptr, merged, tiny, small, big, totals, bsums, bytes;
 };
-RowLayout row_layout(int64_t outer_n, int64_t nnz_p) {
+RowLayout row_layout(int64_t outer_n) {
     RowLayout R;
     Carver cv(nullptr);
-    R.L = cv.reserve<uint32_t>(nnz_p + 1);
     R.cnt = cv.reserve<uint32_t>(outer_n + 2);
     R.cptr = cv.reserve<uint32_t>(outer_n + 2);
     R.tiny = cv.reserve<uint32_t>(outer_n > 0 ? outer_n : 1);
     R.small = cv.reserve<uint32_t>(outer_n > 0 ? outer_n : 1);
     R.big = cv.reserve<uint32_t>(outer_n > 0 ? outer_n : 1);
-    R.counters = cv.reserve<uint32_t>(4);
-    R.totals = cv.reserve<unsigned long long>(2);
-    const int64_t ns = nnz_p + 1 > outer_n + 2 ? nnz_p + 1 : outer_n + 2;
-    R.bsums = cv.reserve<uint32_t>(scan_block_sums(ns));
+    R.merged = cv.reserve<uint32_t>(ceil_div(outer_n, 32) + 1);
+    R.totals = cv.reserve<RowTotals>(1);
+    R.bsums = cv.reserve<uint32_t>(scan_block_sums(outer_n + 2));
     R.bytes = align_up(cv.off, 256);
     return R;
 }
@@ -578,46 +715,39 @@ int read_back(cudaStream_t s, void *host, const void *dev, size_t bytes, const c
 
 // Symbolic phase: counts, row pointers (written to ptr_c), big-row sums.
 template <typename V, typename I>
-int spgemm_create(cudaStream_t s, gsa_spgemm *h, int64_t nnz_p, I *ptr_c) {
+int spgemm_create(cudaStream_t s, gsa_spgemm *h, I *ptr_c) {
     const I *pp = (const I *)h->pp, *pi = (const I *)h->pi, *qp = (const I *)h->qp, *qi = (const I *)h->qi;
     const V *pv = (const V *)h->pv, *qv = (const V *)h->qv;
     const int64_t outer_n = h->outer_n;
-    const RowLayout R = row_layout(outer_n, nnz_p);
-    int rc = check_cuda(cudaMalloc(&h->mem, R.bytes), "spgemm: row arrays");
+    const RowLayout R = row_layout(outer_n);
+    int rc = check_cuda(scratch_alloc(&h->mem, R.bytes, s), "spgemm: row arrays");
     if (rc) return rc;
     char *m = (char *)h->mem;
-    uint32_t *L = (uint32_t *)(m + R.L), *cnt = (uint32_t *)(m + R.cnt), *cptr = (uint32_t *)(m + R.cptr);
+    uint32_t *cnt = (uint32_t *)(m + R.cnt), *cptr = (uint32_t *)(m + R.cptr), *merged = (uint32_t *)(m + R.merged);
     uint32_t *tiny = (uint32_t *)(m + R.tiny), *small = (uint32_t *)(m + R.small), *big = (uint32_t *)(m + R.big);
-    uint32_t *counters = (uint32_t *)(m + R.counters), *bsums = (uint32_t *)(m + R.bsums);
-    unsigned long long *totals = (unsigned long long *)(m + R.totals);
-    h->cnt_off = R.cnt;
+    uint32_t *bsums = (uint32_t *)(m + R.bsums);
+    RowTotals *totals = (RowTotals *)(m + R.totals);
+    uint32_t *counters = totals->counters;
     h->cptr_off = R.cptr;
+    h->merged_off = R.merged;
     h->tiny_off = R.tiny;
     h->small_off = R.small;
     h->big_off = R.big;
-    h->counters_off = R.counters;
-    rc = check_cuda(cudaMemsetAsync(counters, 0, 4 * sizeof(uint32_t), s), "spgemm: clear");
-    if (!rc) rc = check_cuda(cudaMemsetAsync(totals, 0, 2 * sizeof(unsigned long long), s), "spgemm: clear");
-    if (!rc) rc = check_cuda(cudaMemsetAsync(cnt, 0, (size_t)(outer_n + 2) * sizeof(uint32_t), s), "spgemm: clear");
-    if (rc) return rc;
-    entry_flops_kernel<I><<<sg_grid(nnz_p + 1, 256, 152 * 32), 256, 0, s>>>(nnz_p, pi, qp, h->q_outer, h->base, L,
-                                                                            totals);
-    rc = check_cuda(cudaGetLastError(), "spgemm: entry_flops_kernel");
-    unsigned long long tot[2] = {0, 0};
-    if (!rc) rc = read_back(s, tot, totals, sizeof(tot), "spgemm: product count");
-    if (rc) return rc;
-    if (tot[0] >= 0xffffffffull)
-        return fail(GSA_ERR_UNSUPPORTED, "the product has %llu products; at most 2^32 - 2 are supported", tot[0]);
-    rc = scan_u32(s, L, L, nnz_p + 1, bsums);
+    h->counters_off = (size_t)((char *)counters - m);
+    rc = check_cuda(cudaMemsetAsync(totals, 0, sizeof(RowTotals), s), "spgemm: clear");
+    if (!rc) rc = check_cuda(cudaMemsetAsync(cnt + outer_n, 0, 2 * sizeof(uint32_t), s), "spgemm: clear");
     if (rc) return rc;
     if (outer_n > 0)
-        row_flops_kernel<I><<<sg_grid(outer_n, 256, 152 * 32), 256, 0, s>>>(outer_n, pp, h->base, L, cnt, tiny, small, big,
-                                                                          counters, totals);
-    rc = check_cuda(cudaGetLastError(), "spgemm: row_flops_kernel");
-    uint32_t ctr[4] = {0, 0, 0, 0};
-    if (!rc) rc = read_back(s, ctr, counters, sizeof(ctr), "spgemm: row lists");
-    if (!rc) rc = read_back(s, tot, totals, sizeof(tot), "spgemm: big-row products");
+        count_rows_kernel<I><<<sg_grid(outer_n, SG_THREADS, 152 * 64), SG_THREADS, 0, s>>>(
+            outer_n, pp, pi, qp, qi, h->q_outer, h->base, cnt, merged, tiny, small, big, totals);
+    rc = check_cuda(cudaGetLastError(), "spgemm: count_rows_kernel");
+    RowTotals got{};
+    if (!rc) rc = read_back(s, &got, totals, sizeof(got), "spgemm: product counts");
     if (rc) return rc;
+    const unsigned long long *tot = got.totals;
+    const uint32_t *ctr = got.counters;
+    if (tot[0] >= 0xffffffffull)
+        return fail(GSA_ERR_UNSUPPORTED, "the product has %llu products; at most 2^32 - 2 are supported", tot[0]);
     h->nsmall = ctr[0];
     h->nbig = ctr[1];
     h->ntiny = ctr[2];
@@ -634,7 +764,7 @@ int spgemm_create(cudaStream_t s, gsa_spgemm *h, int64_t nnz_p, I *ptr_c) {
     if (rc) return rc;
     if (h->nbig) {
         const BigLayout B = big_layout(h->nbig, h->pbig, sizeof(V));
-        rc = check_cuda(cudaMalloc(&h->big, B.bytes), "spgemm: big-row arrays");
+        rc = check_cuda(scratch_alloc(&h->big, B.bytes, s), "spgemm: big-row arrays");
         if (rc) return rc;
         char *g = (char *)h->big;
         h->flags_off = B.flags;
@@ -650,8 +780,7 @@ int spgemm_create(cudaStream_t s, gsa_spgemm *h, int64_t nnz_p, I *ptr_c) {
         uint64_t *exkey;
         uint32_t *expos;
         radix_sort_inputs(g + B.sort, (int64_t)h->pbig, &exkey, &expos);
-        big_flops_kernel<I><<<sg_grid((int64_t)h->nbig + 1, 256, 152 * 8), 256, 0, s>>>(big, h->nbig, pp, h->base, L,
-                                                                                       bflops);
+        big_flops_kernel<<<sg_grid((int64_t)h->nbig + 1, 256, 152 * 8), 256, 0, s>>>(big, h->nbig, cnt, bflops);
         rc = check_cuda(cudaGetLastError(), "spgemm: big_flops_kernel");
         if (!rc) rc = scan_u32(s, bflops, boff, (int64_t)h->nbig + 1, gbsums);
         if (rc) return rc;
@@ -696,6 +825,10 @@ int spgemm_compute(cudaStream_t s, const gsa_spgemm *h, I *idx_c, V *val_c) {
     const uint32_t *small = (const uint32_t *)(m + h->small_off), *big = (const uint32_t *)(m + h->big_off);
     const uint32_t *tiny = (const uint32_t *)(m + h->tiny_off);
     const uint32_t *counters = (const uint32_t *)(m + h->counters_off);
+    if (h->outer_n > 0)
+        merge_rows_kernel<V, I><<<(unsigned)ceil_div(h->outer_n, SG_THREADS), SG_THREADS, 0, s>>>(
+            h->outer_n, (const uint32_t *)(m + h->merged_off), (const I *)h->pp, (const I *)h->pi, (const V *)h->pv,
+            (const I *)h->qp, (const I *)h->qi, (const V *)h->qv, h->q_outer, h->base, h->csr != 0, cptr, idx_c, val_c);
     if (h->ntiny)
         tiny_kernel<V, I, true><<<sg_grid(h->ntiny, SG_TINY_WARPS * 32, 152 * 32), SG_TINY_WARPS * 32, 0, s>>>(
             tiny, counters, (const I *)h->pp, (const I *)h->pi, (const V *)h->pv, (const I *)h->qp, (const I *)h->qi,
@@ -724,10 +857,9 @@ bool sg_misaligned(const void *p, size_t a) { return a && ((uintptr_t)p % a) != 
 struct SpgemmCreateBody {
     cudaStream_t s;
     gsa_spgemm *h;
-    int64_t nnz_p;
     void *ptr_c;
     template <typename V, typename I> int operator()() {
-        return gsa::spgemm_create<V, I>(s, h, nnz_p, (I *)ptr_c);
+        return gsa::spgemm_create<V, I>(s, h, (I *)ptr_c);
     }
 };
 struct SpgemmComputeBody {
@@ -744,12 +876,8 @@ extern "C" {
 
 int gsa_spgemm_destroy(gsa_spgemm *handle) {
     if (!handle) return GSA_OK;
-    int rc = GSA_OK;
-    if (handle->big) rc = gsa::check_cuda(cudaFree(handle->big), "spgemm: free");
-    if (handle->mem) {
-        const int rc2 = gsa::check_cuda(cudaFree(handle->mem), "spgemm: free");
-        if (!rc) rc = rc2;
-    }
+    const int rc = gsa::scratch_free_after(handle->device, handle->used, {handle->mem, handle->big});
+    if (handle->used) cudaEventDestroy(handle->used);
     delete handle;
     return rc;
 }
@@ -766,7 +894,7 @@ int gsa_spgemm_create(void *stream, int format, int dtype, int itype, int64_t m,
     *handle = nullptr;
     if (m < 0 || k < 0 || n < 0 || nnz_a < 0 || nnz_b < 0) return fail(GSA_ERR_INVALID_ARG, "negative size");
     const bool csr = format == 0;
-    const int64_t outer_n = csr ? m : n, width = csr ? n : m, nnz_p = csr ? nnz_a : nnz_b;
+    const int64_t outer_n = csr ? m : n, width = csr ? n : m;
     if (outer_n >= 0xfffffffeLL || width > 0x100000000LL || k >= 0xfffffffeLL)
         return fail(GSA_ERR_UNSUPPORTED, "dimensions beyond 2^32 - 2 are not supported");
     if (!ptr_a || !ptr_b || !ptr_c) return fail(GSA_ERR_INVALID_ARG, "pointer arrays are NULL");
@@ -789,10 +917,20 @@ int gsa_spgemm_create(void *stream, int format, int dtype, int itype, int64_t m,
     h->qp = csr ? ptr_b : ptr_a;
     h->qi = csr ? idx_b : idx_a;
     h->qv = csr ? val_b : val_a;
-    SpgemmCreateBody body{(cudaStream_t)stream, h, nnz_p, ptr_c};
-    const int rc = dispatch_vi(dtype, itype, body);
+    SpgemmCreateBody body{(cudaStream_t)stream, h, ptr_c};
+    int rc = check_cuda(cudaGetDevice(&h->device), "spgemm: device");
+    if (!rc) rc = check_cuda(cudaEventCreateWithFlags(&h->used, cudaEventDisableTiming), "spgemm: event");
+    if (!rc) rc = dispatch_vi(dtype, itype, body);
+    // (an event that could not be recorded sends the handle's memory through a synchronization)
+    if (h->used && cudaEventRecord(h->used, (cudaStream_t)stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaEventDestroy(h->used);
+        h->used = nullptr;
+    }
     if (rc) {
+        const std::string why = gsa_last_error_string();
         gsa_spgemm_destroy(h);
+        set_error("%s", why.c_str());
         return rc;
     }
     *nnz_c = h->nnz_c;
@@ -808,7 +946,13 @@ int gsa_spgemm_compute(void *stream, gsa_spgemm *handle, void *idx_c, void *val_
     if (sg_misaligned(idx_c, itype_size(handle->itype)) || sg_misaligned(val_c, dtype_size(handle->dtype)))
         return fail(GSA_ERR_INVALID_ARG, "arrays must be aligned to their element size");
     SpgemmComputeBody body{(cudaStream_t)stream, handle, idx_c, val_c};
-    return dispatch_vi(handle->dtype, handle->itype, body);
+    const int rc = dispatch_vi(handle->dtype, handle->itype, body);
+    if (handle->used && cudaEventRecord(handle->used, (cudaStream_t)stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaEventDestroy(handle->used);
+        handle->used = nullptr;
+    }
+    return rc;
 }
 
 }  // extern "C"
