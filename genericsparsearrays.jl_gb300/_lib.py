@@ -107,6 +107,8 @@ class GSAError(RuntimeError):
 def load() -> ctypes.CDLL:
     """Load libgsa.so (built by ``build.py``); raises if it is missing."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):
@@ -118,7 +120,7 @@ def load() -> ctypes.CDLL:
                 fn = getattr(lib, name)
                 fn.argtypes = args
                 fn.restype = res
-            _lib = lib
+            _lib = lib  # only once every signature is set
     return _lib
 
 

@@ -40,6 +40,7 @@ _DTYPE = {torch.float32: _lib.F32, torch.float64: _lib.F64, torch.complex64: _li
 _ITYPE = {torch.int32: _lib.IDX32, torch.int64: _lib.IDX64}
 _NP_OF = {torch.float32: np.float32, torch.float64: np.float64, torch.complex64: np.complex64,
           torch.complex128: np.complex128, torch.int32: np.int32, torch.int64: np.int64}
+_COMPLEX = (torch.complex64, torch.complex128)
 _IMAX = {torch.int32: 2**31 - 1, torch.int64: 2**63 - 1}
 
 # Index base of every buffer this layer creates or accepts (Julia's).
@@ -502,6 +503,105 @@ def _coo_plan(A) -> Optional[_PlanHandle]:
     return A._plan
 
 
+# alpha and beta buffers of -1, 0 and 1 (Python ints), read by the library during the call only
+_SMALL = {(dt, v): np.array([v], dtype=npdt) for dt, npdt in _NP_OF.items() for v in (-1, 0, 1)}
+_SMALL_PTR = {key: buf.ctypes.data for key, buf in _SMALL.items()}
+
+
+def _mul_plain(C, A, B, alpha, beta) -> bool:
+    """The usual call of mul_, or False with nothing done: a matrix (or its transpose / adjoint) whose
+    plan has been made, plain tensors on its device -- the current one -- of its element type, and
+    vectors or column-major matrices of sizes that agree.  Everything else, the errors among it, is
+    mul_'s.  It asks for the same things in fewer Python calls: a product of a small matrix waited 32
+    us for its host code, most of it device and stream objects, ctypes wrappers and scalar arrays."""
+    op, P = _lib.OP_N, A
+    if isinstance(A, Transpose):
+        P = A.parent
+        op = _lib.OP_C if type(A) is Adjoint and getattr(P, "dtype", None) in _COMPLEX else _lib.OP_T
+    cls = type(P)
+    if cls is GenericSparseMatrixCSR:
+        p0, p1 = P.rowptr, P.colval
+    elif cls is GenericSparseMatrixCSC:
+        p0, p1 = P.colptr, P.rowval
+    elif cls is GenericSparseMatrixCOO:
+        p0, p1 = P.rowind, P.colind
+    else:
+        return False
+    plan = P.__dict__.get("_plan", False)
+    if plan is False or type(B) is not torch.Tensor or type(C) is not torch.Tensor:
+        return False
+    val, dt = P.nzval, C.dtype
+    code, icode = _DTYPE.get(dt), _ITYPE.get(p0.dtype)
+    if code is None or icode is None or val.dtype != dt or B.dtype != dt or B.is_conj():
+        return False
+    dev = C.get_device()
+    if dev < 0 or B.get_device() != dev or val.get_device() != dev or dev != torch.cuda.current_device():
+        return False
+    shape = B.shape
+    if len(shape) == 1:
+        r, k = shape[0], 1
+        ldb = r
+        if r > 1 and B.stride(0) != 1:
+            return False
+    elif len(shape) == 2:
+        r, k = shape
+        if r > 1 and B.stride(0) != 1:
+            return False
+        ldb = B.stride(1) if k > 1 else r
+    else:
+        return False
+    shape = C.shape
+    if len(shape) == 1:
+        rc, kc = shape[0], 1
+        ldc = rc
+        if rc > 1 and C.stride(0) != 1:
+            return False
+    elif len(shape) == 2:
+        rc, kc = shape
+        if rc > 1 and C.stride(0) != 1:
+            return False
+        ldc = C.stride(1) if kc > 1 else rc
+    else:
+        return False
+    m, n = P.m, P.n
+    if (m, n, k) != ((rc, r, kc) if op == _lib.OP_N else (r, rc, kc)):
+        return False
+    al = _SMALL_PTR.get((dt, alpha)) if type(alpha) is int else None
+    be = _SMALL_PTR.get((dt, beta)) if type(beta) is int else None
+    if al is None:
+        al_buf = _scalar_buf(alpha, dt)
+        al = al_buf.ctypes.data
+    if be is None:
+        be_buf = _scalar_buf(beta, dt)
+        be = be_buf.ctypes.data
+    lib = _lib.load()
+    stream = _raw_stream(dev)
+    head = (stream, code, icode, m, n, val.numel(), p0.data_ptr(), p1.data_ptr(), val.data_ptr(), BASE, op, k,
+            B.data_ptr(), max(ldb, r, 1), _lib.OP_N, C.data_ptr(), max(ldc, rc, 1), al, be)
+    if plan is not None:
+        size = lib.gsa_plan_workspace_size(plan.handle, code, k)
+        ws = torch.empty(size, dtype=torch.uint8, device=C.device) if size else None
+        fn = (lib.gsa_csr_mul_planned if cls is GenericSparseMatrixCSR else
+              lib.gsa_csc_mul_planned if cls is GenericSparseMatrixCSC else lib.gsa_coo_mul_planned)
+        st = fn(*head, plan.handle, ws.data_ptr() if size else None, size)
+    elif cls is GenericSparseMatrixCOO:
+        st = lib.gsa_coo_mul(*head)
+    else:  # without a plan neither direction takes a workspace
+        fn = lib.gsa_csr_mul if cls is GenericSparseMatrixCSR else lib.gsa_csc_mul
+        st = fn(*head, _lib.ALGO_AUTO, None, 0)
+    if st:
+        _lib.check(st)
+    return True
+
+
+def _raw_stream(dev: int) -> int:
+    return torch.cuda.current_stream(dev).cuda_stream
+
+
+if hasattr(torch._C, "_cuda_getCurrentRawStream"):  # the same number without the stream object
+    _raw_stream = torch._C._cuda_getCurrentRawStream
+
+
 def mul_(C: torch.Tensor, A, B, alpha=1, beta=0, algo: int = _lib.ALGO_AUTO,
          workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``mul!(C, A, B, α, β)``: ``C = β C + α op(A) op(B)`` on the GPU; returns ``C``.
@@ -510,6 +610,8 @@ def mul_(C: torch.Tensor, A, B, alpha=1, beta=0, algo: int = _lib.ALGO_AUTO,
     three ``DimensionMismatch`` checks, the element-type check and the backend check, in that
     order.  ``beta == 0`` never reads ``C``.  Asynchronous on the current torch stream.
     """
+    if algo == _lib.ALGO_AUTO and workspace is None and _mul_plain(C, A, B, alpha, beta):
+        return C
     Ap, opA = _unwrap_sparse(A)
     if not isinstance(Ap, AbstractGenericSparseMatrix):
         raise ArgumentError("A must be a GenericSparseMatrixCSR/CSC/COO or its transpose/adjoint")
