@@ -133,15 +133,23 @@ plan_stats_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int b
             if (all[t]) atomicAdd(&s_sum[3 + t], (unsigned long long)all[t]);
     }
     __syncthreads();
+    // the only CTA writes its sums as they are: no clearing before it
+    const bool alone = gridDim.x == 1;
     if (threadIdx.x == 0) {
-        atomicMax(&totals->max_len, s_sum[0]);
-        atomicAdd(&totals->busy, s_sum[1]);
-        atomicAdd(&totals->held, s_sum[2]);
+        if (alone) {
+            *totals = PlanTotals{s_sum[0], s_sum[1], s_sum[2]};
+        } else {
+            atomicMax(&totals->max_len, s_sum[0]);
+            atomicAdd(&totals->busy, s_sum[1]);
+            atomicAdd(&totals->held, s_sum[2]);
+        }
         counts[blockIdx.x] = PlanCount{{s_sum[3], s_sum[4]}, {s_sum[5], s_sum[6]}};
     }
     uint32_t *h = hist + (r0 / BIN_SEGMENT) * NBINS;
-    for (int b = threadIdx.x; b < NBINS; b += PL_THREADS)
-        if (s_hist[b]) atomicAdd(&h[b], s_hist[b]);
+    for (int b = threadIdx.x; b < NBINS; b += PL_THREADS) {
+        if (alone) h[b] = s_hist[b];
+        else if (s_hist[b]) atomicAdd(&h[b], s_hist[b]);
+    }
 }
 
 // First chunked row and first chunk of each CTA's 4096 rows.
@@ -297,7 +305,7 @@ int build_plan(cudaStream_t s, int64_t outer_n, int64_t nnz, const I *ptr, int b
         int rc = tmp.acquire(s, nullptr, 0, bytes1);
         if (rc) return rc;
         char *d = (char *)tmp.p;
-        rc = check_cuda(cudaMemsetAsync(d, 0, zeroed, s), "plan: clear");
+        if (nct > 1) rc = check_cuda(cudaMemsetAsync(d, 0, zeroed, s), "plan: clear");
         if (rc) return rc;
         plan_stats_kernel<I><<<(unsigned)nct, PL_THREADS, 0, s>>>(outer_n, nnz, ptr, base, (PlanTotals *)(d + o_tot),
                                                                   (PlanCount *)(d + o_cnt), (uint32_t *)(d + o_hist));
