@@ -66,8 +66,13 @@ template <class VT> __host__ __device__ constexpr size_t carried_size() {
     return std::is_same<VT, NoValue>::value ? 0 : sizeof(VT);
 }
 // Entries of a coarse bucket that fine_kernel stages in shared memory, a key each and with values
-// the number of its record: 105 KB, so that two CTAs fit an SM beside the offsets of 1024 rows.
-template <class VT> __host__ __device__ constexpr int stage_entries() { return carried_size<VT>() ? 10496 : 12288; }
+// the number of its record: twice an average bucket's, at most 105 KB, so that two CTAs fit an SM
+// beside the offsets of 1024 rows.  What shared memory leaves caches the records whose values are
+// fetched last (power-law ComplexF64: 395 us with 41 KB staged, 490 with 105 KB).
+template <class VT> inline int stage_entries(int64_t nnz, int64_t nb) {
+    const int64_t most = carried_size<VT>() ? 10496 : 12288, twice = 2 * (nnz / (nb > 1 ? nb - 1 : 1) + 1);
+    return (int)((twice < 2048 ? 2048 : (twice < most ? twice : most)) + 15) & ~15;
+}
 
 struct Coarse {
     bool ok;
@@ -367,8 +372,8 @@ coarse_place_kernel(Src src, int64_t nnz, int64_t first, int64_t major_n, Coarse
 
 // Dynamic shared memory of fine_kernel: the staged keys, row offsets and fill counters for 2^cs
 // rows, and (with values) the record of each key.
-template <class VT> inline size_t fine_smem_bytes(int cs) {
-    return (size_t)stage_entries<VT>() * (8 + (carried_size<VT>() ? 2 : 0)) + (((size_t)2 << cs) + 2) * sizeof(uint32_t);
+template <class VT> inline size_t fine_smem_bytes(int cs, int stage) {
+    return (size_t)stage * (8 + (carried_size<VT>() ? 2 : 0)) + (((size_t)2 << cs) + 2) * sizeof(uint32_t);
 }
 
 // CTA per coarse bucket, taken from a queue (counters[2]): rows counted and scanned in shared
@@ -386,19 +391,17 @@ template <class VT> inline size_t fine_smem_bytes(int cs) {
 // Longer rows are copied out for the kernels of longer rows.
 template <class VT, class Emit>
 __global__ void __launch_bounds__(PC_THREADS, 2)
-fine_kernel(int64_t major_n, Coarse co, const uint32_t *__restrict__ cstart, const Rec<VT> *__restrict__ rec1,
-            uint64_t *key2, VT *val2, uint32_t *__restrict__ start, LongRows longs, Emit emit) {
+fine_kernel(int64_t major_n, Coarse co, int stage, const uint32_t *__restrict__ cstart,
+            const Rec<VT> *__restrict__ rec1, uint64_t *key2, VT *val2, uint32_t *__restrict__ start, LongRows longs, Emit emit) {
     constexpr bool HAS_VAL = !std::is_same<VT, NoValue>::value;
     const int cs = co.cs;
     const int64_t nb = co.nb;
     const int rshift = co.mb + co.pb;  // the row inside the bucket sits above minor and position
     const PackedEmit<Emit> pemit{emit, co.mb, co.pb};
-    constexpr int STAGE = stage_entries<VT>();
-    static_assert(STAGE <= 65536, "16-bit record numbers");
     constexpr int ITEMS = ROWS_MAX / PC_THREADS;
     extern __shared__ __align__(16) unsigned char dsm[];
     uint64_t *s_key = (uint64_t *)dsm;
-    uint32_t *s_off = (uint32_t *)(s_key + STAGE);
+    uint32_t *s_off = (uint32_t *)(s_key + stage);
     const int rmax = 1 << cs;
     uint32_t *s_fill = s_off + rmax + 1;  // counts, then fill cursors
     uint16_t *s_src = (uint16_t *)(s_fill + rmax + 1);
@@ -413,7 +416,7 @@ fine_kernel(int64_t major_n, Coarse co, const uint32_t *__restrict__ cstart, con
         const int64_t row0 = invalid ? major_n : bk << cs;
         const int64_t rspan = major_n - row0 < (int64_t)rmax ? major_n - row0 : (int64_t)rmax;
         const int R = invalid ? 1 : (int)rspan;
-        const bool staged = E <= (uint32_t)STAGE;
+        const bool staged = E <= (uint32_t)stage;
         for (int j = threadIdx.x; j < R; j += PC_THREADS) s_fill[j] = 0;
         if (threadIdx.x == 0) {
             s_next = (int64_t)gridDim.x + atomicAdd(&longs.counters[2], 1u);
@@ -531,10 +534,11 @@ fine_kernel(int64_t major_n, Coarse co, const uint32_t *__restrict__ cstart, con
 constexpr int ST_THREADS = 1024;
 constexpr int FS_MAXI = 8;                   // pass C: at most 8 staged records per thread
 constexpr int STAGE_ROW_AVG = 8;             // pass C staged while rows average at most 8 entries
-// Pass C staged: a thread sorts rows of up to 8 entries in place, a warp rows of 9 to 256.  (A
-// 16-key in-place thread sort, which at this kernel's 64 registers runs mostly from spilled
-// registers, left rows of 9 to 16 entries unsorted and corrupted the index array on GB300; the
-// warp sort takes those rows.)
+// Pass C staged: a thread sorts rows of up to 8 entries in place; the entries of rows of 9 to 256
+// find their places by counting, as in fine_kernel.  (A warp per such row, and the bucket waiting
+// for its longest, took 1374 us for 2M rows of Poisson(7) lengths against 599, and 605 against 391 for
+// Poisson(5).  A 16-key in-place thread sort, which at this kernel's 64 registers ran mostly from
+// spilled registers, left rows of 9 to 16 entries unsorted and corrupted the index array on GB300.)
 constexpr int STAGE_SMALL = 8;
 
 // The CTA copies the bytes [src, src + bytes) to dst, both 16-byte aligned, in 16-byte
@@ -576,38 +580,6 @@ template <class R> __device__ __forceinline__ void sort_idx_short(const R *rec, 
     if (len <= 4) sort_idx_registers<R, 4>(rec, idx, len);
     else sort_idx_registers<R, STAGE_SMALL>(rec, idx, len);
 }
-// A warp sorts the record indices of one row of up to WARP_MAX entries in place: each lane
-// holds up to 8 keys, and every key is compared with the row's keys broadcast 32 at a time.
-template <class R> __device__ __forceinline__ void sort_idx_warp(const R *rec, uint16_t *idx, uint32_t len, int lane) {
-    constexpr int P = WARP_MAX / 32;
-    uint64_t k[P];
-    uint32_t ix[P], rank[P];
-#pragma unroll
-    for (int m = 0; m < P; ++m) {
-        const uint32_t t = (uint32_t)(m * 32 + lane);
-        ix[m] = t < len ? idx[t] : 0u;
-        k[m] = t < len ? rec[ix[m]].key : ~0ull;
-        rank[m] = 0;
-    }
-#pragma unroll
-    for (int g = 0; g < P; ++g) {
-        if ((uint32_t)(g * 32) >= len) break;  // uniform across the warp
-        for (int l = 0; l < 32; ++l) {
-            const uint64_t kl = __shfl_sync(0xffffffffu, k[g], l);
-#pragma unroll
-            for (int m = 0; m < P; ++m)
-                if ((uint32_t)(m * 32) < len) rank[m] += kl < k[m] ? 1u : 0u;
-        }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int m = 0; m < P; ++m) {
-        const uint32_t t = (uint32_t)(m * 32 + lane);
-        if (t < len) idx[rank[m]] = (uint16_t)ix[m];
-    }
-    __syncwarp();
-}
-
 // Pass C's buffer: the most records per bucket whose two buffers and index array fit beside
 // the row offsets and counters (a multiple of 16, at most FS_MAXI * ST_THREADS).
 template <class VT> inline int fine_stage_cap(int cs, size_t smem_max) {
@@ -623,9 +595,9 @@ template <class VT> inline size_t fine_stage_smem(int cs, int cap) {
 
 // Pass C, staged: one CTA per SM takes buckets from a queue (counters[2]) and copies the
 // next bucket's records into shared memory while it sorts the current one.  Rows are
-// counted, scanned (the row pointers) and placed as record indices; rows of up to 16
-// entries are sorted by a thread, up to 256 by a warp, longer ones listed for the kernels of longer rows;
-// then the bucket's output is written in order.  A bucket of more than `cap` entries takes
+// counted, scanned (the row pointers) and placed as record indices; rows of up to 8
+// entries are sorted by a thread, the entries of rows of up to 256 count their places, longer
+// rows are listed for the kernels of longer rows; then the bucket's output is written.  A bucket of more than `cap` entries takes
 // fine_kernel's global path (rows placed into key2 / val2, then sorted there or listed).
 template <class VT, class Emit>
 __global__ void __launch_bounds__(ST_THREADS, 1)
@@ -643,9 +615,9 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
     uint16_t *s_idx = (uint16_t *)(s_buf + 2 * (size_t)cap);
     uint32_t *s_off = (uint32_t *)(s_idx + cap);
     const int rmax = 1 << cs;
-    uint32_t *s_cnt = s_off + rmax + 1;  // row counts; then fill cursors (global path) or the warp row list
+    uint32_t *s_cnt = s_off + rmax + 1;  // row counts; then fill cursors (global path)
     __shared__ uint32_t s_warp[ST_THREADS / 32];
-    __shared__ uint32_t s_nlist, s_long;
+    __shared__ uint32_t s_mid, s_long;  // whether the bucket has rows of 9 to 256 entries, longer ones
     __shared__ int64_t s_next;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int64_t bk = blockIdx.x;
@@ -665,7 +637,7 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
         for (int j = threadIdx.x; j < R; j += ST_THREADS) s_cnt[j] = 0;
         if (threadIdx.x == 0) {
             s_next = (int64_t)gridDim.x + atomicAdd(&longs.counters[2], 1u);
-            s_nlist = 0;
+            s_mid = 0;
             s_long = 0;
         }
         __syncthreads();
@@ -760,25 +732,28 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
                     const uint32_t o = s_off[j];
                     len = s_off[j + 1] - o;
                     if (len <= (uint32_t)STAGE_SMALL) sort_idx_short(s_rec, s_idx + o, len);
-                    else if (len <= (uint32_t)WARP_MAX) s_cnt[atomicAdd(&s_nlist, 1u)] = (uint32_t)j;
+                    else if (len <= (uint32_t)WARP_MAX) s_mid = 1;
                 }
                 list_long_rows(valid && len > (uint32_t)WARP_MAX, len, (uint32_t)(row0 + j), longs);
             }
             __syncthreads();
-            if (s_nlist) {  // uniform
-                for (uint32_t q = warp; q < s_nlist; q += ST_THREADS / 32) {
-                    const uint32_t j = s_cnt[q];
-                    const uint32_t o = s_off[j];
-                    sort_idx_warp(s_rec, s_idx + o, s_off[j + 1] - o, lane);
-                }
-                __syncthreads();
-            }
+            const bool mid = s_mid != 0;  // uniform
             // the bucket's output in order (longer rows are rewritten by their kernels)
             for (uint32_t p = threadIdx.x; p < E; p += ST_THREADS) {
                 const Rec<VT> r = s_rec[s_idx[p]];
-                const uint64_t row = (uint64_t)row0 + shr64(r.key, rshift);
-                if constexpr (HAS_VAL) pemit.put(B0 + p, row, r.key, r.val);
-                else pemit.gather(B0 + p, row, r.key);
+                const uint32_t lrow = (uint32_t)shr64(r.key, rshift);
+                uint32_t at = p;
+                if (mid) {
+                    const uint32_t o = s_off[lrow], len = s_off[lrow + 1] - o;
+                    if (len > (uint32_t)STAGE_SMALL && len <= (uint32_t)WARP_MAX) {
+                        at = o;
+#pragma unroll 4
+                        for (uint32_t u = 0; u < len; ++u) at += s_rec[s_idx[o + u]].key < r.key ? 1u : 0u;
+                    }
+                }
+                const uint64_t row = (uint64_t)row0 + lrow;
+                if constexpr (HAS_VAL) pemit.put(B0 + at, row, r.key, r.val);
+                else pemit.gather(B0 + at, row, r.key);
             }
         } else {
             __syncthreads();  // the fill cursors are zero
@@ -875,12 +850,29 @@ warp_kernel(const uint32_t *__restrict__ start, const uint64_t *__restrict__ key
     }
 }
 
+// The smaller (or larger) of lane l's and lane l ^ j's key.
+__device__ __forceinline__ uint64_t exchange(uint64_t x, int j, bool smaller) {
+    const uint64_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    return (x < y) == smaller ? x : y;
+}
+
 // Bitonic sort of s[0 .. P), P a power of two of at least 32, by the CTA.  Distances below 32 are
 // exchanged by shuffles (element i is in lane i mod 32 of whichever warp holds it), one pass and
 // barrier for all of a stage's: 36 barriers for 4096 keys instead of 78.
 __device__ __forceinline__ void bitonic_shared(uint64_t *s, uint32_t P) {
     const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t k = 32; k <= P; k <<= 1) {
+    for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {  // whole warps: P is a multiple of 32
+        uint64_t x = s[i];
+#pragma unroll
+        for (int lk = 1; lk <= 5; ++lk) {
+            const bool up = (i & (1u << lk)) == 0;
+#pragma unroll
+            for (int lj = lk - 1; lj >= 0; --lj) x = exchange(x, 1 << lj, ((lane & (1u << lj)) == 0) == up);
+        }
+        s[i] = x;
+    }
+    __syncthreads();
+    for (uint32_t k = 64; k <= P; k <<= 1) {
         for (uint32_t j = k >> 1; j >= 32; j >>= 1) {
             for (uint32_t t = threadIdx.x; t < P / 2; t += blockDim.x) {
                 const uint32_t i = 2 * t - (t & (j - 1));
@@ -892,17 +884,11 @@ __device__ __forceinline__ void bitonic_shared(uint64_t *s, uint32_t P) {
             }
             __syncthreads();
         }
-        for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {  // whole warps: P is a multiple of 32
+        for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
             uint64_t x = s[i];
-            // the first pass sorts every 32 keys from scratch
-            for (uint32_t kk = k == 32 ? 2 : k; kk <= k; kk <<= 1) {
-                const bool up = (i & kk) == 0;
-                for (uint32_t j = kk >> 1 < 16 ? kk >> 1 : 16; j > 0; j >>= 1) {
-                    const uint64_t y = __shfl_xor_sync(0xffffffffu, x, j);
-                    const bool low = (lane & j) == 0;
-                    x = (x < y) == (low == up) ? x : y;
-                }
-            }
+            const bool up = (i & k) == 0;
+#pragma unroll
+            for (int lj = 4; lj >= 0; --lj) x = exchange(x, 1 << lj, ((lane & (1u << lj)) == 0) == up);
             s[i] = x;
         }
         __syncthreads();
@@ -917,17 +903,20 @@ __device__ __forceinline__ void bitonic_shared(uint64_t *s, uint32_t P) {
 //
 // A row's chunks are spread over the SMs, so the longest row sets no tail: one CTA per row, chunk
 // sorts, pairwise merges and all, took 1.0 to 1.2 ms for the power-law matrix of 10^6 rows, one SM
-// busy with its row of 50,000 entries all that time, against 0.2 (sort) and 0.1 ms (merge).  The work of a row grows with the square of
+// busy with its row of 50,000 entries all that time, against 0.12 (sort) and 0.07 ms
+// (merge).  The work of a row grows with the square of
 // its chunks, and stays below the pairwise merges' up to rows of some 10^8 entries.
 template <class Emit>
 __global__ void __launch_bounds__(LONG_THREADS)
 long_sort_kernel(const uint32_t *__restrict__ start, uint64_t *keys, LongRows longs, Emit emit) {
     __shared__ uint64_t s[LONG_CHUNK];
+    __shared__ uint32_t s_next;
     const uint32_t nitems = longs.counters[1];
-    for (uint32_t q = blockIdx.x; q < nitems; q += gridDim.x) {
+    for (uint32_t q = blockIdx.x; q < nitems;) {  // from a queue (counters[3]): chunks differ 16-fold
         const uint2 item = longs.items[q];
         const uint32_t b = start[item.x], len = start[item.x + 1] - b, c0 = item.y * LONG_CHUNK;
         const uint32_t n = len - c0 < (uint32_t)LONG_CHUNK ? len - c0 : (uint32_t)LONG_CHUNK;
+        if (threadIdx.x == 0) s_next = gridDim.x + atomicAdd(&longs.counters[3], 1u);
         uint32_t P = 32;
         while (P < n) P <<= 1;
         for (uint32_t j = threadIdx.x; j < P; j += LONG_THREADS) s[j] = j < n ? keys[b + c0 + j] : ~0ull;
@@ -937,6 +926,7 @@ long_sort_kernel(const uint32_t *__restrict__ start, uint64_t *keys, LongRows lo
             if (len <= (uint32_t)LONG_CHUNK) emit.gather(b + j, (uint64_t)item.x, s[j]);
             else keys[b + c0 + j] = s[j];
         }
+        q = s_next;
         __syncthreads();
     }
 }
@@ -961,22 +951,39 @@ long_merge_kernel(const uint32_t *__restrict__ start, const uint64_t *__restrict
             rank[u] = j;
         }
         const uint32_t nchunks = (len - 1) / LONG_CHUNK + 1;
-        for (uint32_t d = 0; d < nchunks; ++d) {
-            if (d == item.y) continue;
-            const uint32_t d0 = d * LONG_CHUNK;
-            const uint32_t m = len - d0 < (uint32_t)LONG_CHUNK ? len - d0 : (uint32_t)LONG_CHUNK;
-            for (uint32_t j = threadIdx.x; j < m; j += LONG_THREADS) s[j] = keys[b + d0 + j];
-            __syncthreads();
+        auto size_of = [&](uint32_t d) {
+            const uint32_t left = len - d * LONG_CHUNK;
+            return left < (uint32_t)LONG_CHUNK ? left : (uint32_t)LONG_CHUNK;
+        };
+        uint64_t ahead[PER];  // the next chunk, read while the current one is searched
+        auto read = [&](uint32_t d) {
+            const uint32_t m = size_of(d);
 #pragma unroll
             for (int u = 0; u < PER; ++u) {
-                uint32_t lo = 0, hi = m;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (s[mid] < k[u]) lo = mid + 1;
-                    else hi = mid;
-                }
-                rank[u] += lo;
+                const uint32_t j = (uint32_t)(u * LONG_THREADS) + threadIdx.x;
+                ahead[u] = j < m ? keys[b + d * LONG_CHUNK + j] : ~0ull;
             }
+        };
+        uint32_t d = item.y == 0 ? 1u : 0u;
+        read(d);  // the row has another chunk
+        while (d < nchunks) {
+            const uint32_t m = size_of(d);
+#pragma unroll
+            for (int u = 0; u < PER; ++u) s[u * LONG_THREADS + threadIdx.x] = ahead[u];
+            __syncthreads();
+            d += d + 1 == item.y ? 2u : 1u;
+            if (d < nchunks) read(d);
+            // smaller keys of the chunk, all of a thread's keys one step at a time
+            uint32_t at[PER];
+#pragma unroll
+            for (int u = 0; u < PER; ++u) at[u] = 0;
+            for (uint32_t step = LONG_CHUNK; step > 0; step >>= 1) {
+#pragma unroll
+                for (int u = 0; u < PER; ++u)
+                    if (at[u] + step <= m && s[at[u] + step - 1] < k[u]) at[u] += step;
+            }
+#pragma unroll
+            for (int u = 0; u < PER; ++u) rank[u] += at[u];
             __syncthreads();
         }
 #pragma unroll
@@ -1073,13 +1080,14 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
                 major_n, co, fcap, cstart, rec1, key2, val2, start, longs, emit);
             return launch_long_rows<VT, Emit>(s, start, key2, val2, longs, emit);
         }
-        const size_t smem = fine_smem_bytes<VT>(co.cs);
+        const int stage = stage_entries<VT>(nnz, co.nb);
+        const size_t smem = fine_smem_bytes<VT>(co.cs, stage);
         rc = check_cuda(cudaFuncSetAttribute(fine_kernel<VT, Emit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem),
                         "bucket: fine_kernel shared memory");
         if (rc) return rc;
         fine_kernel<VT, Emit><<<grid_for(co.nb, 1, 152 * 2), PC_THREADS, smem, s>>>(
-            major_n, co, cstart, rec1, key2, val2, start, longs, emit);
+            major_n, co, stage, cstart, rec1, key2, val2, start, longs, emit);
         return launch_long_rows<VT, Emit>(s, start, key2, val2, longs, emit);
     }
     src.parts([&](const auto &part, int64_t n, int64_t) {
