@@ -2,12 +2,12 @@
 //
 // What a plan holds is described at gsa_plan (gsa_internal.cuh).  Making it is three passes over
 // the row pointers, which they are bound by (8 B per row at most; 10^6 rows: tens of
-// microseconds), with the few numbers per 4096 rows that set the sizes worked out on the host in
+// microseconds), with the few numbers per 2048 rows that set the sizes worked out on the host in
 // between:
-//   1. plan_stats_kernel: per 4096 rows the chunked rows and chunks of both sets; over all rows the
+//   1. plan_stats_kernel: per 2048 rows the chunked rows and chunks of both sets; over all rows the
 //      longest row and how much of the natural order's lanes would be busy; per segment the rows
 //      of each bin.
-//   2. the host sums the 4096-row counts into offsets and lays out groups and warps.
+//   2. the host sums the 2048-row counts into offsets and lays out groups and warps.
 //   3. chunk_set_kernel writes a set's rows, chunks and mask; bin_order_kernel a segment's rows by
 //      bin, stable, and its warps' groups.
 // The same work on the host, one thread over a copy of the pointers, took 8.5 ms for 10^6 rows of
@@ -23,7 +23,7 @@ namespace {
 
 constexpr int PL_THREADS = 256;
 constexpr int PL_WARPS = PL_THREADS / 32;
-constexpr int64_t PL_ROWS = 4096;       // rows per CTA of the counting and chunk passes
+constexpr int64_t PL_ROWS = 2048;       // rows per CTA of the counting and chunk passes
 constexpr int64_t BIN_SEGMENT = 32768;  // rows per segment of the bin order
 constexpr int BO_THREADS = 1024;
 constexpr int BO_WARPS = BO_THREADS / 32;
@@ -71,7 +71,7 @@ __device__ __forceinline__ int64_t warp_sum(int64_t v) {
 struct PlanTotals {
     unsigned long long max_len, busy, held;
 };
-// Chunked rows and their chunks of one CTA's 4096 rows, per set.
+// Chunked rows and their chunks of one CTA's 2048 rows, per set.
 struct PlanCount {
     unsigned long long rows[2], chunks[2];
 };
@@ -152,18 +152,31 @@ plan_stats_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int b
     }
 }
 
-// First chunked row and first chunk of each CTA's 4096 rows.
+// First chunked row and first chunk of each CTA's 2048 rows.
 struct PlanFirst {
     int64_t row, chunk;
 };
 
-// Rows, chunks and mask of set t, in row order: a CTA's 4096 rows in steps of 256, each step's
-// places from a scan over the CTA's warps.
+// One set's arrays as chunk_set_kernel writes them.
+struct PlanSet {
+    const PlanFirst *firsts;
+    int64_t *row;
+    int32_t *first, *count, *chunk_slot;
+    uint32_t *mask;
+};
+
+// Rows, chunks and mask of set t = blockIdx.y, in row order: a CTA's 2048 rows in steps of 256, each
+// step's places from a scan over the CTA's warps.
 template <typename I>
 __global__ void __launch_bounds__(PL_THREADS)
-chunk_set_kernel(int t, int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int base,
-                 const PlanFirst *__restrict__ firsts, int64_t *__restrict__ row, int32_t *__restrict__ first,
-                 int32_t *__restrict__ count, int32_t *__restrict__ chunk_slot, uint32_t *__restrict__ mask) {
+chunk_set_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int base, PlanSet natural, PlanSet binned) {
+    const int t = blockIdx.y;
+    const PlanSet &set = t == 0 ? natural : binned;
+    const PlanFirst *__restrict__ firsts = set.firsts;
+    int64_t *__restrict__ row = set.row;
+    int32_t *__restrict__ first = set.first, *__restrict__ count = set.count;
+    int32_t *__restrict__ chunk_slot = set.chunk_slot;
+    uint32_t *__restrict__ mask = set.mask;
     __shared__ int64_t s_rows[PL_WARPS], s_chunks[PL_WARPS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int64_t at_row = firsts[blockIdx.x].row, at_chunk = firsts[blockIdx.x].chunk;
@@ -397,22 +410,23 @@ int build_plan(cudaStream_t s, int64_t outer_n, int64_t nnz, const I *ptr, int b
     }
     rc = check_cuda(cudaMemcpyAsync(d, host.data(), uploaded, cudaMemcpyHostToDevice, s), "plan: upload");
     if (rc) return rc;
-    for (int t = 0; t < (binned ? 2 : 1); ++t) {
+    PlanSet sets[2];
+    for (int t = 0; t < 2; ++t) {
+        sets[t] = PlanSet{(const PlanFirst *)(d + o_first[t]), (int64_t *)(d + o_row[t]), (int32_t *)(d + o_cfirst[t]),
+                          (int32_t *)(d + o_count[t]), (int32_t *)(d + o_slot[t]), (uint32_t *)(d + o_mask[t])};
         gsa_chunk_set &c = t == 0 ? p->nat : p->bin;
         c.nlong = nlong[t];
         c.nchunks = nchunks[t];
-        c.row = (const int64_t *)(d + o_row[t]);
-        c.first = (const int32_t *)(d + o_cfirst[t]);
-        c.count = (const int32_t *)(d + o_count[t]);
-        c.chunk_slot = (const int32_t *)(d + o_slot[t]);
-        c.skip_mask = (const uint32_t *)(d + o_mask[t]);
-        chunk_set_kernel<I><<<(unsigned)nct, PL_THREADS, 0, s>>>(
-            t, outer_n, nnz, ptr, base, (const PlanFirst *)(d + o_first[t]), (int64_t *)(d + o_row[t]),
-            (int32_t *)(d + o_cfirst[t]), (int32_t *)(d + o_count[t]), (int32_t *)(d + o_slot[t]),
-            (uint32_t *)(d + o_mask[t]));
-        rc = check_cuda(cudaGetLastError(), "chunk_set_kernel");
-        if (rc) return rc;
+        c.row = sets[t].row;
+        c.first = sets[t].first;
+        c.count = sets[t].count;
+        c.chunk_slot = sets[t].chunk_slot;
+        c.skip_mask = sets[t].mask;
     }
+    chunk_set_kernel<I><<<dim3((unsigned)nct, binned ? 2 : 1), PL_THREADS, 0, s>>>(outer_n, nnz, ptr, base, sets[0],
+                                                                                  sets[1]);
+    rc = check_cuda(cudaGetLastError(), "chunk_set_kernel");
+    if (rc) return rc;
     if (binned) {
         bin_order_kernel<I><<<(unsigned)nseg, BO_THREADS, 0, s>>>(
             outer_n, nnz, ptr, base, (const PlanSegment *)(d + o_segs), (const int64_t *)(d + o_groups),

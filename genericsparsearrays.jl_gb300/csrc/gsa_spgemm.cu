@@ -12,7 +12,7 @@
 //      selects; a row of many entries by its whole warp), and counts the entries of rows of at most
 //      8 entries and 32 products at once by merging their Q rows, which sorted rows allow: the
 //      smallest next column, its products in order, the next.  merge_rows_kernel walks the same
-//      merges again for the values and writes 32 neighbouring rows together.  The other rows are
+//      merges again for the values, 32 neighbouring rows in step, and writes them together.  The other rows are
 //      listed as tiny, small or big.
 //   2. listed tiny rows (at most 32 products, unsorted or of more than 8 entries), a thread each
 //      (tiny_kernel), and small rows (at most
@@ -57,7 +57,7 @@ namespace {
 constexpr int SG_TINY_P = 32;     // products a thread sums in shared memory
 constexpr int SG_TINY_WARPS = 2;
 constexpr int SG_TINY_A = 8;      // entries of a merged row (their loads are issued together)
-constexpr int SG_MERGE_OUT = 16;  // entries of a merged row that are written together with its neighbours'
+constexpr int SG_MERGE_OUT = 8;   // entries of a merged row that are written together with its neighbours'
 constexpr int SG_WARP_P = 256;    // products a warp sums in shared memory
 constexpr int SG_THREADS = 128;   // 4 warps
 constexpr int SG_WARPS = SG_THREADS / 32;
@@ -93,60 +93,61 @@ struct RowTotals {
     uint32_t counters[4];
 };
 
-// The Q rows that up to SG_TINY_A entries of a row select, as cursors: entry c's row is at
-// cur[c], len[c] entries (0: none).  Returns the products.
-template <typename I>
+// The Q rows that up to K entries of a row select, as cursors: entry c's row is [cur[c], end[c]).
+// Returns the products.
+template <typename I, int K>
 __device__ __forceinline__ uint64_t open_rows(const I *__restrict__ pi, const I *__restrict__ qp, int64_t q_outer, int base,
-                                              int64_t b, int n, Off<I> (&cur)[SG_TINY_A], uint32_t (&len)[SG_TINY_A]) {
-    int64_t k[SG_TINY_A];
+                                              int64_t b, int n, Off<I> (&cur)[K], Off<I> (&end)[K]) {
+    int64_t k[K];
 #pragma unroll
-    for (int c = 0; c < SG_TINY_A; ++c) k[c] = c < n ? (int64_t)__ldg(pi + b + c) - base : -1;
+    for (int c = 0; c < K; ++c) k[c] = c < n ? (int64_t)__ldg(pi + b + c) - base : -1;
     uint64_t f = 0;
 #pragma unroll
-    for (int c = 0; c < SG_TINY_A; ++c) {
+    for (int c = 0; c < K; ++c) {
         const bool ok = (uint64_t)k[c] < (uint64_t)q_outer;
         const int64_t q0 = ok ? (int64_t)__ldg(qp + k[c]) - base : 0;
-        len[c] = ok ? (uint32_t)((int64_t)__ldg(qp + k[c] + 1) - base - q0) : 0u;
+        const uint32_t len = ok ? (uint32_t)((int64_t)__ldg(qp + k[c] + 1) - base - q0) : 0u;
         cur[c] = (Off<I>)q0;
-        f += len[c];
+        end[c] = (Off<I>)q0 + (Off<I>)len;
+        f += len;
     }
     return f;
 }
 
 // Merges the open rows of a row of at most SG_TINY_P products: visit(j) for every column j in
 // increasing order after take(c, at) for each of its products in the reference's order (entries in
-// order, each Q row in order).  False, with part of them visited, when a Q row is not sorted.  (A
-// second column held per cursor, loaded one advance ahead, was slower: 591 us against 510 for
-// merge_rows_kernel on the 2048^2 grid, for its registers.)
-template <typename I, typename Take, typename Visit>
-__device__ __forceinline__ bool merge_open_rows(const I *__restrict__ qi, int base, Off<I> (&cur)[SG_TINY_A],
-                                                uint32_t (&len)[SG_TINY_A], Take &&take, Visit &&visit) {
+// order, each Q row in order).  False, with part of them visited, when a Q row is not sorted, or has
+// the column that the end mark stands for.  Bound by its instructions: K is 5 for the warps whose
+// rows have no more entries (a grid's): 212 us against 250 with 8 for count_rows_kernel on the 2048^2 grid.
+// (A second column held per cursor, loaded one advance ahead, was slower: 591 us against 510 for
+// merge_rows_kernel, for its registers.)
+template <typename I, int K, typename Take, typename Visit>
+__device__ __forceinline__ bool merge_open_rows(const I *__restrict__ qi, int base, Off<I> (&cur)[K], Off<I> (&end)[K],
+                                                Take &&take, Visit &&visit) {
     constexpr uint32_t END = 0xffffffffu;
-    uint32_t jc[SG_TINY_A];
+    const uint32_t ubase = (uint32_t)base;
+    uint32_t jc[K];
     bool sorted = true;
 #pragma unroll
-    for (int c = 0; c < SG_TINY_A; ++c) {
-        jc[c] = len[c] ? (uint32_t)((int64_t)__ldg(qi + cur[c]) - base) : END;
-        if (len[c] && jc[c] == END) sorted = false;  // a column that the end mark cannot stand beside
+    for (int c = 0; c < K; ++c) {
+        jc[c] = cur[c] < end[c] ? (uint32_t)__ldg(qi + cur[c]) - ubase : END;
+        if (cur[c] < end[c] && jc[c] == END) sorted = false;
     }
     for (int guard = 0; sorted && guard <= SG_TINY_P; ++guard) {
         uint32_t jmin = jc[0];
 #pragma unroll
-        for (int c = 1; c < SG_TINY_A; ++c) jmin = jc[c] < jmin ? jc[c] : jmin;
+        for (int c = 1; c < K; ++c) jmin = jc[c] < jmin ? jc[c] : jmin;
         if (jmin == END) break;
 #pragma unroll
-        for (int c = 0; c < SG_TINY_A; ++c) {
+        for (int c = 0; c < K; ++c) {
             while (jc[c] == jmin) {
                 take(c, cur[c]);
                 ++cur[c];
-                if (--len[c]) {
-                    jc[c] = (uint32_t)((int64_t)__ldg(qi + cur[c]) - base);
-                    if (jc[c] < jmin || jc[c] == END) {
-                        sorted = false;
-                        jc[c] = END;
-                    }
-                } else {
-                    jc[c] = END;
+                jc[c] = END;
+                if (cur[c] < end[c]) {
+                    const uint32_t j = (uint32_t)__ldg(qi + cur[c]) - ubase;
+                    if (j + 1u <= jmin) sorted = false;  // smaller, or the end mark's
+                    else jc[c] = j;
                 }
             }
         }
@@ -155,10 +156,16 @@ __device__ __forceinline__ bool merge_open_rows(const I *__restrict__ qi, int ba
     return sorted;
 }
 
+// Calls f(K) for the smallest K that covers the warp's rows of n entries each.
+template <typename F> __device__ __forceinline__ void by_entries(int n, F &&f) {
+    if (__reduce_max_sync(0xffffffffu, (unsigned)n) <= 5u) f(std::integral_constant<int, 5>{});
+    else f(std::integral_constant<int, SG_TINY_A>{});
+}
+
 // A lane per row (of 32 neighbouring ones per warp): products, and for rows that merge_rows_kernel
 // takes (a bit in merged) their entries, into cnt; big rows leave their products there.  Bound by
 // the merges' instructions (issue slots 75 % busy).  The 2048^2 grid's
-// 105M products: 250 us; a flop count per stored entry, a scan of all of them, a pass over the rows
+// 105M products: 212 us; a flop count per stored entry, a scan of all of them, a pass over the rows
 // and tiny_kernel's symbolic pass took 665.
 template <typename I>
 __global__ void __launch_bounds__(SG_THREADS)
@@ -181,9 +188,19 @@ count_rows_kernel(int64_t outer_n, const I *__restrict__ pp, const I *__restrict
             n = (int64_t)__ldg(pp + o + 1) - base - b;
         }
         const bool few = n <= SG_TINY_A;
-        Off<I> cur[SG_TINY_A];
-        uint32_t len[SG_TINY_A];
-        uint64_t f = open_rows<I>(pi, qp, q_outer, base, b, few ? (int)(n > 0 ? n : 0) : 0, cur, len);
+        const int nf = few ? (int)(n > 0 ? n : 0) : 0;
+        uint64_t f = 0;
+        uint32_t count = 0;
+        bool done = false;
+        auto take_rows = [&](auto kc) {
+            constexpr int K = decltype(kc)::value;
+            Off<I> cur[K], end[K];
+            f = open_rows<I, K>(pi, qp, q_outer, base, b, nf, cur, end);
+            done = f > 0 && f <= (uint64_t)SG_TINY_P;
+            if (done) done = merge_open_rows<I, K>(qi, base, cur, end, [](int, Off<I>) {}, [&](uint32_t) { ++count; });
+        };
+        by_entries(nf, take_rows);
+        __syncwarp();
         for (unsigned todo = __ballot_sync(0xffffffffu, !few); todo; todo &= todo - 1) {  // a row by its whole warp
             const int l = __ffs(todo) - 1;
             const int64_t bl = __shfl_sync(0xffffffffu, b, l), el = bl + __shfl_sync(0xffffffffu, n, l);
@@ -197,10 +214,6 @@ count_rows_kernel(int64_t outer_n, const I *__restrict__ pp, const I *__restrict
             for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
             if (lane == l) f = x;
         }
-        uint32_t count = 0;
-        bool done = few && f > 0 && f <= (uint64_t)SG_TINY_P;
-        if (done) done = merge_open_rows<I>(qi, base, cur, len, [](int, Off<I>) {}, [&](uint32_t) { ++count; });
-        __syncwarp();
         const bool is_tiny = !done && f > 0 && f <= (uint64_t)SG_TINY_P;
         const bool is_small = f > (uint64_t)SG_TINY_P && f <= (uint64_t)SG_WARP_P, is_big = f > (uint64_t)SG_WARP_P;
         if (valid) cnt[o] = done ? count : (is_big ? (uint32_t)f : 0u);
@@ -232,10 +245,14 @@ count_rows_kernel(int64_t outer_n, const I *__restrict__ pp, const I *__restrict
     }
 }
 
-// The entries of the merged rows, a lane per row, 32 neighbouring rows per warp: the warp's rows
-// leave their first SG_MERGE_OUT entries in shared memory and write them together, two rows at a
-// time, as one stretch of the result.  (A thread writing its own row sent every entry as a store
-// of its own, 109M of them for the 2048^2 grid: 940 us against 510.)
+// The entries of the merged rows, a lane per row, 32 neighbouring rows per warp.  The lanes merge in
+// step, one entry each per turn, and leave up to SG_MERGE_OUT entries per row in shared memory; the
+// warp then writes them together, four rows at a time.  (A thread writing its own row sent every
+// entry as a store of its own, 109M of them for the 2048^2 grid: 940 us.)  Bound by the latency of
+// the Q rows' reads, which L1 has to hold (with 16 entries per row in shared memory 14 % of them hit,
+// 510 us; with 8 62 %, 496), and the FP64 pipe: a column's first product is not added to zero but
+// given the bits that gives, 474 us, the pipe 54 % active.  (Values loaded with their columns, a step
+// ahead: 468 us at 80 registers, not taken.)
 template <typename V, typename I>
 __global__ void __launch_bounds__(SG_THREADS)
 merge_rows_kernel(int64_t outer_n, const uint32_t *__restrict__ merged, const I *__restrict__ pp,
@@ -243,6 +260,7 @@ merge_rows_kernel(int64_t outer_n, const uint32_t *__restrict__ merged, const I 
                   const I *__restrict__ qi, const V *__restrict__ qv, int64_t q_outer, int base, bool csr,
                   const uint32_t *__restrict__ cptr, I *__restrict__ idx_out, V *__restrict__ val_out) {
     constexpr int LD = 33;  // slot s of lane l at s * 33 + l: neither phase meets itself in a bank
+    constexpr uint32_t END = 0xffffffffu;
     __shared__ uint32_t s_j[SG_WARPS][SG_MERGE_OUT * LD];
     __shared__ V s_v[SG_WARPS][SG_MERGE_OUT * LD];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -250,47 +268,73 @@ merge_rows_kernel(int64_t outer_n, const uint32_t *__restrict__ merged, const I 
     if (row0 >= outer_n) return;  // the whole warp
     const unsigned md = __ldg(merged + (row0 >> 5));
     if (!md) return;
-    const bool mine = (md >> lane) & 1u;
     const int64_t o = row0 + lane;
-    uint32_t out0 = 0, count = 0;
-    if (mine) {
-        const int64_t b = (int64_t)__ldg(pp + o) - base;
-        const int n = (int)((int64_t)__ldg(pp + o + 1) - base - b);
-        out0 = cptr[o];
-        Off<I> cur[SG_TINY_A];
-        uint32_t len[SG_TINY_A];
-        V a[SG_TINY_A];
-#pragma unroll
-        for (int c = 0; c < SG_TINY_A; ++c) a[c] = c < n ? ldg(pv + b + c) : VT<V>::zero();
-        open_rows<I>(pi, qp, q_outer, base, b, n, cur, len);
-        V acc = VT<V>::zero();
-        merge_open_rows<I>(
-            qi, base, cur, len, [&](int c, Off<I> at) { acc = add(acc, product(a[c], ldg(qv + at), csr)); },
-            [&](uint32_t j) {
-                if (count < (uint32_t)SG_MERGE_OUT) {
-                    s_j[w][count * LD + lane] = j;
-                    s_v[w][count * LD + lane] = acc;
-                } else {
-                    idx_out[out0 + count] = (I)((int64_t)j + base);
-                    val_out[out0 + count] = acc;
-                }
-                ++count;
-                acc = VT<V>::zero();
-            });
+    uint32_t at = 0, held = 0, left = 0;  // the row's next place, its entries in shared memory, entries to come
+    int64_t b = 0;
+    int n = 0;
+    if ((md >> lane) & 1u) {
+        b = (int64_t)__ldg(pp + o) - base;
+        n = (int)((int64_t)__ldg(pp + o + 1) - base - b);
+        at = cptr[o];
+        left = cptr[o + 1] - at;
     }
-    __syncwarp();
-    const uint32_t together = count < (uint32_t)SG_MERGE_OUT ? count : (uint32_t)SG_MERGE_OUT;
-    const int t = lane & (SG_MERGE_OUT - 1);
-    static_assert(SG_MERGE_OUT == 16, "two rows per step of a warp");
+    auto write_held = [&] {
+        __syncwarp();
+        constexpr int ROWS = 32 / SG_MERGE_OUT;
+        const int t = lane % SG_MERGE_OUT;
 #pragma unroll 4
-    for (int l0 = 0; l0 < 32; l0 += 2) {
-        const int l = l0 + (lane >> 4);
-        const uint32_t nl = __shfl_sync(0xffffffffu, together, l), at = __shfl_sync(0xffffffffu, out0, l) + t;
-        if ((uint32_t)t < nl) {
-            idx_out[at] = (I)((int64_t)s_j[w][t * LD + l] + base);
-            val_out[at] = s_v[w][t * LD + l];
+        for (int l0 = 0; l0 < 32; l0 += ROWS) {
+            const int l = l0 + lane / SG_MERGE_OUT;
+            const uint32_t nl = __shfl_sync(0xffffffffu, held, l), to = __shfl_sync(0xffffffffu, at, l) + t;
+            if ((uint32_t)t < nl) {
+                idx_out[to] = (I)((int64_t)s_j[w][t * LD + l] + base);
+                val_out[to] = s_v[w][t * LD + l];
+            }
         }
-    }
+        __syncwarp();
+        at += held;
+        held = 0;
+    };
+    by_entries(n, [&](auto kc) {
+        constexpr int K = decltype(kc)::value;
+        Off<I> cur[K], end[K];
+        V a[K];
+#pragma unroll
+        for (int c = 0; c < K; ++c) a[c] = c < n ? ldg(pv + b + c) : VT<V>::zero();
+        open_rows<I, K>(pi, qp, q_outer, base, b, n, cur, end);
+        uint32_t jc[K];
+#pragma unroll
+        for (int c = 0; c < K; ++c) jc[c] = cur[c] < end[c] ? (uint32_t)__ldg(qi + cur[c]) - (uint32_t)base : END;
+        for (int turn = 1; turn <= SG_TINY_P; ++turn) {  // at most an entry per product
+            uint32_t jmin = jc[0];
+#pragma unroll
+            for (int c = 1; c < K; ++c) jmin = jc[c] < jmin ? jc[c] : jmin;
+            if (left == 0) jmin = END;
+            if (!__any_sync(0xffffffffu, jmin != END)) break;
+            if (jmin != END) {
+                V acc = VT<V>::zero();
+                bool first = true;
+#pragma unroll
+                for (int c = 0; c < K; ++c) {
+                    while (jc[c] == jmin) {
+                        const V x = product(a[c], ldg(qv + cur[c]), csr);
+                        // 0 + x without the FP64 add, where no lane needs one
+                        if (__any_sync(__activemask(), !first)) acc = first ? zero_plus(x) : add(acc, x);
+                        else acc = zero_plus(x);
+                        first = false;
+                        ++cur[c];
+                        jc[c] = cur[c] < end[c] ? (uint32_t)__ldg(qi + cur[c]) - (uint32_t)base : END;
+                    }
+                }
+                s_j[w][held * LD + lane] = jmin;
+                s_v[w][held * LD + lane] = acc;
+                ++held;
+                --left;
+            }
+            if (turn % SG_MERGE_OUT == 0) write_held();
+        }
+    });
+    write_held();
 }
 
 // Thread per listed tiny row (at most SG_TINY_P products): the same expansion, sums and
