@@ -24,10 +24,11 @@ namespace {
 constexpr int PL_THREADS = 256;
 constexpr int PL_WARPS = PL_THREADS / 32;
 constexpr int64_t PL_ROWS = 2048;       // rows per CTA of the counting and chunk passes
+constexpr int64_t PL_ALONE = 8192;      // up to as many rows one CTA takes them all
 constexpr int64_t BIN_SEGMENT = 32768;  // rows per segment of the bin order
 constexpr int BO_THREADS = 1024;
 constexpr int BO_WARPS = BO_THREADS / 32;
-static_assert(BIN_SEGMENT % PL_ROWS == 0, "a counting CTA lies in one segment");
+static_assert(BIN_SEGMENT % PL_ROWS == 0 && PL_ALONE <= BIN_SEGMENT, "a counting CTA lies in one segment");
 static_assert(BIN_SEGMENT % (32 * BO_WARPS) == 0, "a segment's warps take whole groups of 32 rows");
 
 // Bin of a row of len <= CHUNK entries and its lanes per row: rows of equal length up to
@@ -81,7 +82,8 @@ struct PlanCount {
 // it; each of the G passes lasts as long as its longest row).  hist: rows of each bin per segment.
 template <typename I>
 __global__ void __launch_bounds__(PL_THREADS)
-plan_stats_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int base, PlanTotals *__restrict__ totals,
+plan_stats_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int base, int64_t rows,
+                  PlanTotals *__restrict__ totals,
                   PlanCount *__restrict__ counts, uint32_t *__restrict__ hist) {
     __shared__ uint32_t s_hist[NBINS];
     __shared__ unsigned long long s_sum[7];  // max_len, busy, held, rows[2], chunks[2]
@@ -90,9 +92,9 @@ plan_stats_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int b
     __syncthreads();
     const int lane = threadIdx.x & 31;
     int64_t longest = 0, busy = 0, held = 0, nrows[2] = {0, 0}, nchunks[2] = {0, 0};
-    const int64_t r0 = (int64_t)blockIdx.x * PL_ROWS;
+    const int64_t r0 = (int64_t)blockIdx.x * rows;
 #pragma unroll 4
-    for (int64_t w0 = r0 + (threadIdx.x & ~31); w0 < r0 + PL_ROWS; w0 += PL_THREADS) {
+    for (int64_t w0 = r0 + (threadIdx.x & ~31); w0 < r0 + rows; w0 += PL_THREADS) {
         if (w0 >= outer_n) break;  // the whole warp
         const int64_t len = row_length(ptr, base, outer_n, nnz, w0 + lane);
         longest = len > longest ? len : longest;
@@ -169,7 +171,8 @@ struct PlanSet {
 // step's places from a scan over the CTA's warps.
 template <typename I>
 __global__ void __launch_bounds__(PL_THREADS)
-chunk_set_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int base, PlanSet natural, PlanSet binned) {
+chunk_set_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int base, int64_t rows, PlanSet natural,
+                 PlanSet binned) {
     const int t = blockIdx.y;
     const PlanSet &set = t == 0 ? natural : binned;
     const PlanFirst *__restrict__ firsts = set.firsts;
@@ -180,7 +183,7 @@ chunk_set_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int ba
     __shared__ int64_t s_rows[PL_WARPS], s_chunks[PL_WARPS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int64_t at_row = firsts[blockIdx.x].row, at_chunk = firsts[blockIdx.x].chunk;
-    for (int64_t b0 = (int64_t)blockIdx.x * PL_ROWS; b0 < (int64_t)(blockIdx.x + 1) * PL_ROWS; b0 += PL_THREADS) {
+    for (int64_t b0 = (int64_t)blockIdx.x * rows; b0 < (int64_t)(blockIdx.x + 1) * rows; b0 += PL_THREADS) {
         if (b0 >= outer_n) break;  // the whole CTA
         const int64_t w0 = b0 + 32 * w, r = w0 + lane;
         const int64_t len = row_length(ptr, base, outer_n, nnz, r);
@@ -297,11 +300,30 @@ bin_order_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int ba
     }
 }
 
+// Host memory that a kernel writes its few counts to: one page per host thread, which waits for
+// the kernel before it reads, and given back when the thread ends.  NULL where it cannot be had.
+constexpr size_t COUNT_BOX = 4096;
+char *count_box() {
+    struct Box {
+        void *p = nullptr;
+        ~Box() {
+            if (p) cudaFreeHost(p);
+        }
+    };
+    static thread_local Box box;
+    if (!box.p && cudaHostAlloc(&box.p, COUNT_BOX, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        box.p = nullptr;
+    }
+    return (char *)box.p;
+}
+
 template <typename I>
 int build_plan(cudaStream_t s, int64_t outer_n, int64_t nnz, const I *ptr, int base, Plan *p) {
     p->outer_n = outer_n;
     p->nnz = nnz;
-    const int64_t nct = ceil_div(outer_n, PL_ROWS), nseg = ceil_div(outer_n, BIN_SEGMENT);
+    const int64_t rows = outer_n <= PL_ALONE ? PL_ALONE : PL_ROWS;
+    const int64_t nct = ceil_div(outer_n, rows), nseg = ceil_div(outer_n, BIN_SEGMENT);
     if (nct > 0x7fffffffLL) return fail(GSA_ERR_UNSUPPORTED, "plan: too many outer entries");
     if (outer_n == 0) {  // nothing to launch: a plan of no rows (the stream is synchronized as ever)
         return check_cuda(cudaStreamSynchronize(s), "plan: sync");
@@ -312,24 +334,34 @@ int build_plan(cudaStream_t s, int64_t outer_n, int64_t nnz, const I *ptr, int b
     const size_t zeroed = sc.off;
     const size_t o_cnt = sc.reserve<PlanCount>((size_t)nct);
     const size_t bytes1 = sc.off;
-    std::vector<char> got(bytes1);
-    {
+    std::vector<char> copied;
+    const char *got = nullptr;
+    auto count = [&](char *d) {
+        plan_stats_kernel<I><<<(unsigned)nct, PL_THREADS, 0, s>>>(outer_n, nnz, ptr, base, rows, (PlanTotals *)(d + o_tot),
+                                                                  (PlanCount *)(d + o_cnt), (uint32_t *)(d + o_hist));
+        return check_cuda(cudaGetLastError(), "plan_stats_kernel");
+    };
+    if (nct == 1 && bytes1 <= COUNT_BOX && (got = count_box())) {
+        // one CTA: its sums go straight to host memory, without scratch and a copy (30 us a plan with)
+        int rc = count((char *)got);
+        if (!rc) rc = check_cuda(cudaStreamSynchronize(s), "plan: sync");
+        if (rc) return rc;
+    } else {
+        copied.resize(bytes1);
         Workspace tmp;
         int rc = tmp.acquire(s, nullptr, 0, bytes1);
         if (rc) return rc;
         char *d = (char *)tmp.p;
         if (nct > 1) rc = check_cuda(cudaMemsetAsync(d, 0, zeroed, s), "plan: clear");
-        if (rc) return rc;
-        plan_stats_kernel<I><<<(unsigned)nct, PL_THREADS, 0, s>>>(outer_n, nnz, ptr, base, (PlanTotals *)(d + o_tot),
-                                                                  (PlanCount *)(d + o_cnt), (uint32_t *)(d + o_hist));
-        rc = check_cuda(cudaGetLastError(), "plan_stats_kernel");
-        if (!rc) rc = check_cuda(cudaMemcpyAsync(got.data(), d, bytes1, cudaMemcpyDeviceToHost, s), "plan: counts");
+        if (!rc) rc = count(d);
+        if (!rc) rc = check_cuda(cudaMemcpyAsync(copied.data(), d, bytes1, cudaMemcpyDeviceToHost, s), "plan: counts");
         if (!rc) rc = check_cuda(cudaStreamSynchronize(s), "plan: sync");
         if (rc) return rc;
+        got = copied.data();
     }
-    const PlanTotals &tot = *(const PlanTotals *)(got.data() + o_tot);
-    const uint32_t *hist = (const uint32_t *)(got.data() + o_hist);
-    const PlanCount *cnt = (const PlanCount *)(got.data() + o_cnt);
+    const PlanTotals &tot = *(const PlanTotals *)(got + o_tot);
+    const uint32_t *hist = (const uint32_t *)(got + o_hist);
+    const PlanCount *cnt = (const PlanCount *)(got + o_cnt);
     p->max_len = (int64_t)tot.max_len;
     // bin order when the natural one would leave over a tenth of the lanes idle (only
     // FP64-bound products use it, where every idle lane is lost FP64 time)
@@ -423,7 +455,7 @@ int build_plan(cudaStream_t s, int64_t outer_n, int64_t nnz, const I *ptr, int b
         c.chunk_slot = sets[t].chunk_slot;
         c.skip_mask = sets[t].mask;
     }
-    chunk_set_kernel<I><<<dim3((unsigned)nct, binned ? 2 : 1), PL_THREADS, 0, s>>>(outer_n, nnz, ptr, base, sets[0],
+    chunk_set_kernel<I><<<dim3((unsigned)nct, binned ? 2 : 1), PL_THREADS, 0, s>>>(outer_n, nnz, ptr, base, rows, sets[0],
                                                                                   sets[1]);
     rc = check_cuda(cudaGetLastError(), "chunk_set_kernel");
     if (rc) return rc;

@@ -172,7 +172,7 @@ __device__ __forceinline__ void warp_rows(const CompressedArgs<V, I> &a, int64_t
         V acc[KC];
 #pragma unroll
         for (int c = 0; c < KC; ++c) acc[c] = VT<V>::zero();
-        accumulate_range<V, I, KC, G, (G == 1 ? (KC >= 16 ? 2 : GSA_G1_UNROLL) : GSA_GN_UNROLL), LAY>(a, B, qb + (O)(lane % G), qe, c0,
+        accumulate_range<V, I, KC, G, (G == 1 ? (KC >= 16 ? 1 : GSA_G1_UNROLL) : GSA_GN_UNROLL), LAY>(a, B, qb + (O)(lane % G), qe, c0,
                                                                                   k, acc);
         if (G > 1) {
 #pragma unroll
