@@ -298,8 +298,14 @@ template <typename V, typename I>
 int launch_scatter_block(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t k, DenseIn<V> B,
                          DenseOut<V> C, const Plan *plan) {
     const int64_t nrb = ceil_div(a.outer_n, RB_THREADS);
+    // Columns per thread: more share an entry's loads, fewer keep more warps at the atomics that
+    // bound the kernel.  Measured with KC = 2 / 4, us (adjoints, Int32 indices): Poisson(10) rows, n =
+    // 10^5, 5 and 8 columns ComplexF32 37.5 / 42.0 and 52.6 / 60.7, Float64 37.8 / 47.2 and 52.2 / 56.2,
+    // Float32 36.7 / 43.0 and 48.3 / 50.2; 1024^2 grid, 8 columns ComplexF32 91 / 93, Float64 117.5 /
+    // 117.5, Float32 56 / 48; three columns 30.4 / 25.8, 30.6 / 27.5 and 28.7 / 25.5 on the Poisson rows.
+    // Hence 2 for values of 8 bytes and more, 4 for three columns and for 4-byte values.
     int KC = get_spmm_columns();
-    if (KC == 0) KC = sizeof(V) >= 16 ? 2 : 4;
+    if (KC == 0) KC = sizeof(V) >= 16 ? 2 : (sizeof(V) == 8 && k != 3 ? 2 : 4);
     if (k == 1) KC = 1;
     if (KC > k) KC = k <= 2 ? 2 : (k <= 4 ? 4 : 8);
     const int64_t ncg = ceil_div(k, KC);
