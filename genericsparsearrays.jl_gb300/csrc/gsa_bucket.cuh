@@ -123,12 +123,13 @@ constexpr size_t rec_size(size_t vsize) { return vsize == 0 ? 8 : (vsize <= 8 ? 
 template <class VT> __device__ __forceinline__ void store_rec(Rec<VT> *p, uint64_t key, const VT &v) {
     static_assert(sizeof(VT) == 4 || sizeof(VT) == 8 || sizeof(VT) == 16, "record values of 4, 8 or 16 bytes");
     if constexpr (sizeof(VT) == 16) {
-        ulonglong2 head, tail;
-        head.x = key;
-        head.y = 0;
-        memcpy(&tail, &v, 16);
-        reinterpret_cast<ulonglong2 *>(p)[0] = head;
-        reinterpret_cast<ulonglong2 *>(p)[1] = tail;
+        // one 32-byte store (records start on 32-byte boundaries): the scattered stores cost by their
+        // number (two 16-byte ones: the placement of 16.4M ComplexF64 entries 560 us against 338)
+        unsigned long long tail[2];
+        memcpy(tail, &v, 16);
+        asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)), "l"(key), "l"(0ull),
+                     "l"(tail[0]), "l"(tail[1])
+                     : "memory");
     } else {
         ulonglong2 w;
         w.x = key;

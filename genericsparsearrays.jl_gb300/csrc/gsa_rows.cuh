@@ -1,5 +1,5 @@
-// Row-gather device code shared by the plain kernel (gsa_rowblock.cu) and the grouped
-// kernel (gsa_batch.cu): sums over row segments, G lanes per row for a warp's rows.
+// Row-gather device code shared by the plain kernel (gsa_rowblock.cuh) and the grouped
+// kernel (gsa_grouped.cuh): sums over row segments, G lanes per row for a warp's rows.
 #pragma once
 
 #include <type_traits>
