@@ -23,8 +23,9 @@
  * is the k x rows(op(B)) matrix that Julia's Transpose/Adjoint wraps.
  *
  * Workspace: entry points that need scratch take (workspace, workspace_bytes).
- * Pass workspace == NULL to let the library take it from the stream-ordered
- * pool (cudaMallocAsync / cudaFreeAsync on the same stream); otherwise pass at
+ * Pass workspace == NULL to let the library take it from its stream-ordered
+ * pool (one per device, allocated and freed on the same stream; it keeps at most
+ * 256 MB over a synchronization); otherwise pass at
  * least the size the matching *_workspace_size function returns.  A caller
  * workspace must not be used by another call that overlaps on the GPU.
  */
@@ -294,8 +295,9 @@ int gsa_csr_spmv_noalloc(void *stream, int dtype, int itype, int64_t m, int64_t 
  * gives each chunk a warp of its own (a long entry is summed chunk by chunk across
  * the whole GPU) and keeps such entries out of the warps of short ones -- what
  * power-law row lengths need; without such entries a plan changes nothing.
- * Creating one copies the pointer array to the host once and synchronizes the
- * stream; the plan holds one device allocation until destroyed.  The structure
+ * Creating one reads the pointer array on the GPU and synchronizes the stream (the host
+ * sees counts only); the plan holds one device allocation until destroyed, which
+ * synchronizes the device.  The structure
  * must not change while its plan is in use.  No counterpart in the reference (its
  * kernels take one work item per row). */
 typedef struct gsa_plan gsa_plan;
