@@ -649,18 +649,25 @@ template int launch_validate<int64_t>(cudaStream_t, int64_t, int64_t, int64_t, c
 // first loads.
 
 // Clears *sorted where a row index decreases or lies outside [base, base + m).  Bound by the read
-// of the indices; a warp leaves once any warp has found a violation.
+// of the indices; a warp leaves once any warp has found a violation, and writes its own once (every
+// thread of a COO in random order writing the one word took 390 us).
 template <typename I>
 __global__ void coo_sorted_kernel(int64_t nnz, const I *__restrict__ rowind, int base, int64_t m,
                                   volatile int *sorted) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < nnz; i0 += stride) {
-        if (!*sorted) return;
+        if (!__any_sync(0xffffffffu, *sorted != 0)) return;
         const int64_t i = i0 + threadIdx.x;
-        if (i >= nnz) return;
-        const int64_t cur = (int64_t)rowind[i] - base;
-        const int64_t prev = i == 0 ? 0 : (int64_t)rowind[i - 1] - base;
-        if (cur < prev || cur < 0 || cur >= m) *sorted = 0;
+        bool bad = false;
+        if (i < nnz) {
+            const int64_t cur = (int64_t)rowind[i] - base;
+            const int64_t prev = i == 0 ? 0 : (int64_t)rowind[i - 1] - base;
+            bad = cur < prev || cur < 0 || cur >= m;
+        }
+        if (__any_sync(0xffffffffu, bad)) {
+            if ((threadIdx.x & 31) == 0) *sorted = 0;
+            return;
+        }
     }
 }
 
@@ -694,7 +701,8 @@ static int coo_row_pointers_i(cudaStream_t s, int64_t m, int64_t nnz, const I *r
                               int *flag, int *sorted_host) {
     int64_t blocks = ceil_div(nnz + 1, 256);
     if (blocks > 152 * 64) blocks = 152 * 64;
-    if (nnz > 0) coo_sorted_kernel<I><<<(unsigned)blocks, 256, 0, s>>>(nnz, rowind, base, m, flag);
+    const int64_t check = blocks < 152 * 8 ? blocks : 152 * 8;  // one wave: the rest would start to leave
+    if (nnz > 0) coo_sorted_kernel<I><<<(unsigned)check, 256, 0, s>>>(nnz, rowind, base, m, flag);
     int rc = check_cuda(cudaGetLastError(), "coo_sorted_kernel");
     if (!rc) rc = check_cuda(cudaMemcpyAsync(sorted_host, flag, sizeof(int), cudaMemcpyDeviceToHost, s),
                              "coo plan: flag");

@@ -36,10 +36,10 @@ namespace gsa {
 // values are latency-bound gathers whose speed follows the warps in flight, so they are
 // held to 32 registers (16 CTAs of 128 threads, every warp slot of the SM).  So are, less tightly,
 // the kernels of many columns of a column-major B, whose loads in flight otherwise take up to 128
-// registers (2048^2 grid; us unbounded / held): Float32 KC = 16 at 48 registers 250 / 161 (64: 167), KC = 8 at
-// 48 270 / 205, KC = 2 at 40 66 / 59 (32 registers spill: Poisson(10) rows 87 against 81), ComplexF32 KC = 8 at 64 202 / 168.  Float64 KC = 8, taken for longer rows, is the
-// faster unbounded (Poisson(10) rows 383 against 453).  0 leaves the register count to the
-// compiler.
+// registers (2048^2 grid; us unbounded / held): Float32 KC = 16 at 48 registers 250 / 161 (64: 167),
+// KC = 8 at 48 270 / 205, KC = 2 at 40 66 / 59 (32 registers spill: Poisson(10) rows 87 against 81),
+// ComplexF32 KC = 8 at 64 202 / 168.  Float64 KC = 8, taken for longer rows, is the faster unbounded
+// (Poisson(10) rows 383 against 453).  0 leaves the register count to the compiler.
 #ifndef GSA_RB_MIN_BLOCKS
 #define GSA_RB_MIN_BLOCKS 16
 #endif
