@@ -29,6 +29,7 @@
 // P and Q: CSR C = A * B runs over A's rows (P = A, Q = B); CSC C = A * B over B's columns
 // (P = B, Q = A).  Products are A-value times B-value with Julia's arithmetic (separate
 // multiply and add, textbook complex product), so the sums are the reference's bit for bit.
+#include <mutex>
 #include <string>
 #include <type_traits>
 
@@ -45,7 +46,10 @@ struct gsa_spgemm {
     void *mem = nullptr;        // per-row arrays
     void *big = nullptr;        // big-row expansion and sort
     int device = 0;             // of both
-    cudaEvent_t used = nullptr; // after the handle's last work
+    cudaEvent_t used = nullptr; // after the handle's work so far, which is all on one stream
+    std::mutex lock;            // of what follows
+    unsigned long long stream = 0;
+    bool any = false, many = false;  // work on a stream; work that `used` cannot cover
     size_t cptr_off = 0, tiny_off = 0, small_off = 0, big_off = 0, counters_off = 0, merged_off = 0;
     size_t boff_off = 0, keys_off = 0, flags_off = 0, rpos_off = 0, sums_off = 0;
     int cb = 0;                 // column bits of the big-row sort keys
@@ -916,11 +920,30 @@ struct SpgemmComputeBody {
 };
 }  // namespace
 
+// After work of the handle on stream s: `used` covers it while all of it is on one stream and runs
+// now.  Work on a second stream and captured work (its graph runs when the program says) are
+// covered by no one event, and what cannot be told or recorded by none: the handle's memory then
+// goes through a synchronization of the device.
+static void spgemm_used(gsa_spgemm *h, cudaStream_t s) {
+    std::lock_guard<std::mutex> hold(h->lock);
+    if (h->many) return;
+    unsigned long long id = 0;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool plain = h->used && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+                       cudaStreamGetId(s, &id) == cudaSuccess && (!h->any || id == h->stream) &&
+                       cudaEventRecord(h->used, s) == cudaSuccess;
+    if (!plain) cudaGetLastError();
+    h->many = !plain;
+    h->any = true;
+    h->stream = id;
+}
+
 extern "C" {
 
 int gsa_spgemm_destroy(gsa_spgemm *handle) {
     if (!handle) return GSA_OK;
-    const int rc = gsa::scratch_free_after(handle->device, handle->used, {handle->mem, handle->big});
+    const int rc = gsa::scratch_free_after(handle->device, handle->many ? nullptr : handle->used,
+                                           {handle->mem, handle->big});
     if (handle->used) cudaEventDestroy(handle->used);
     delete handle;
     return rc;
@@ -965,12 +988,7 @@ int gsa_spgemm_create(void *stream, int format, int dtype, int itype, int64_t m,
     int rc = check_cuda(cudaGetDevice(&h->device), "spgemm: device");
     if (!rc) rc = check_cuda(cudaEventCreateWithFlags(&h->used, cudaEventDisableTiming), "spgemm: event");
     if (!rc) rc = dispatch_vi(dtype, itype, body);
-    // (an event that could not be recorded sends the handle's memory through a synchronization)
-    if (h->used && cudaEventRecord(h->used, (cudaStream_t)stream) != cudaSuccess) {
-        cudaGetLastError();
-        cudaEventDestroy(h->used);
-        h->used = nullptr;
-    }
+    spgemm_used(h, (cudaStream_t)stream);
     if (rc) {
         const std::string why = gsa_last_error_string();
         gsa_spgemm_destroy(h);
@@ -991,11 +1009,7 @@ int gsa_spgemm_compute(void *stream, gsa_spgemm *handle, void *idx_c, void *val_
         return fail(GSA_ERR_INVALID_ARG, "arrays must be aligned to their element size");
     SpgemmComputeBody body{(cudaStream_t)stream, handle, idx_c, val_c};
     const int rc = dispatch_vi(handle->dtype, handle->itype, body);
-    if (handle->used && cudaEventRecord(handle->used, (cudaStream_t)stream) != cudaSuccess) {
-        cudaGetLastError();
-        cudaEventDestroy(handle->used);
-        handle->used = nullptr;
-    }
+    spgemm_used(handle, (cudaStream_t)stream);
     return rc;
 }
 

@@ -253,8 +253,10 @@ int gsa_compressed_add_copy(void *stream, int dtype, int itype, int64_t outer_n,
  * _create runs the symbolic phase: it returns the entry count in *nnz_c (synchronizing the
  * stream to read it) and then writes C's pointer array ptr_c (m + 1 for CSR, n + 1 for CSC)
  * on the stream; the handle keeps device scratch and refers to A's and B's arrays, which must
- * stay unchanged until _compute.  _compute writes idx_c / val_c (nnz_c each).  _destroy frees
- * the handle.  At most 2^32 - 2 products (stored A entries times the lengths of the B rows
+ * stay unchanged until _compute.  _compute writes idx_c / val_c (nnz_c each); it may run on
+ * another stream than _create, more than once, and under capture.  _destroy frees the handle: its
+ * memory stays until the work enqueued before has finished, for which _destroy waits (for the
+ * whole device) if that work was on several streams or captured.  At most 2^32 - 2 products (stored A entries times the lengths of the B rows
  * they select); with Int32 indices at most 2^31 - 1 - base entries (GSA_ERR_UNSUPPORTED, and
  * ptr_c untouched, beyond that). */
 typedef struct gsa_spgemm gsa_spgemm;
