@@ -106,9 +106,9 @@ inline Coarse coarse_plan(int64_t major_n, int64_t minor_n, int64_t nnz, int sta
 }
 
 // Pass B's record: the packed key and the carried value, stored together (one 16- or 32-byte
-// store per entry).
+// store per entry, to which the record is aligned).
 template <class VT, bool HAS = !std::is_same<VT, NoValue>::value> struct Rec;
-template <class VT> struct alignas(16) Rec<VT, true> {
+template <class VT> struct alignas(sizeof(VT) == 16 ? 32 : 16) Rec<VT, true> {
     uint64_t key;
     VT val;
 };
@@ -400,7 +400,7 @@ fine_kernel(int64_t major_n, Coarse co, int stage, const uint32_t *__restrict__ 
     const int rshift = co.mb + co.pb;  // the row inside the bucket sits above minor and position
     const PackedEmit<Emit> pemit{emit, co.mb, co.pb};
     constexpr int ITEMS = ROWS_MAX / PC_THREADS;
-    extern __shared__ __align__(16) unsigned char dsm[];
+    extern __shared__ __align__(32) unsigned char dsm[];
     uint64_t *s_key = (uint64_t *)dsm;
     uint32_t *s_off = (uint32_t *)(s_key + stage);
     const int rmax = 1 << cs;
@@ -611,7 +611,7 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
     const int64_t nb = co.nb;
     const int rshift = co.mb + co.pb;
     const PackedEmit<Emit> pemit{emit, co.mb, co.pb};
-    extern __shared__ __align__(16) unsigned char dsm[];
+    extern __shared__ __align__(32) unsigned char dsm[];
     Rec<VT> *s_buf = (Rec<VT> *)dsm;  // two buffers of cap records
     uint16_t *s_idx = (uint16_t *)(s_buf + 2 * (size_t)cap);
     uint32_t *s_off = (uint32_t *)(s_idx + cap);
@@ -1009,7 +1009,8 @@ inline unsigned grid_for(int64_t n, int64_t per_cta, int64_t cap) {
     return (unsigned)(b > 0 ? b : 1);
 }
 
-// The whole sort.  VT: the type of the values to carry, which the parts give (NoValue: none).
+// The whole sort, on a workspace of layout(...).bytes that starts on a 256-byte boundary where values are
+// carried (8-byte where none are).  VT: the type of the values to carry, which the parts give (NoValue: none).
 // scan(s, in, out, n, bsums) is the library's exclusive scan of uint32.
 template <class VT, class Src, class Emit, class Scan>
 int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Src &src, const Emit &emit, void *ws,

@@ -417,12 +417,17 @@ int radix_sort_pairs(cudaStream_t s, void *ws, int64_t n, int total_bits, uint64
 }
 int radix_bits_for(int64_t count) { return bits_for(count); }
 
+// A caller's workspace may start anywhere; the layouts place their regions from a boundary that
+// the bucket sort's 32-byte records (and all else) can lie on.
+constexpr size_t CALLER_ALIGN = 256;
+
 template <typename V, typename I>
 size_t coo_to_compressed_workspace_size(int64_t m, int64_t n, int64_t nnz, bool colmajor) {
     if (nnz == 0) return 0;
     const int64_t major_n = colmajor ? n : m, minor_n = colmajor ? m : n;
-    if (bucket_fits(major_n, minor_n, nnz)) return bucket::layout(major_n, minor_n, nnz, sizeof(V), SC_TILE).bytes;
-    return sort_layout(nnz).bytes;
+    return CALLER_ALIGN + (bucket_fits(major_n, minor_n, nnz)
+                               ? bucket::layout(major_n, minor_n, nnz, sizeof(V), SC_TILE).bytes
+                               : sort_layout(nnz).bytes);
 }
 
 template <typename V, typename I>
@@ -485,9 +490,10 @@ int launch_coo_to_compressed(cudaStream_t s, bool colmajor, int64_t m, int64_t n
         pointer_kernel<I><<<1, 256, 0, s>>>(0, nullptr, minor_bits, major_n, base, ptr_out);
         return check_cuda(cudaGetLastError(), "pointer_kernel");
     }
+    if (ws_bytes < coo_to_compressed_workspace_size<V, I>(m, n, nnz, colmajor))
+        return fail(GSA_ERR_INVALID_ARG, "conversion workspace too small");
+    ws = (void *)align_up((size_t)ws, CALLER_ALIGN);
     if (bucket_fits(major_n, minor_n, nnz)) {
-        if (ws_bytes < bucket::layout(major_n, minor_n, nnz, sizeof(V), SC_TILE).bytes)
-            return fail(GSA_ERR_INVALID_ARG, "conversion workspace too small");
         const PairSource<V, I> src{major, minor, val, base, nnz};
         CompressedEmit<V, I> emit{ptr_out, idx_out, val_out, val, base, major_n, nnz};
         timer_before(s);
@@ -496,7 +502,6 @@ int launch_coo_to_compressed(cudaStream_t s, bool colmajor, int64_t m, int64_t n
         return rc;
     }
     SortLayout L = sort_layout(nnz);
-    if (ws_bytes < L.bytes) return fail(GSA_ERR_INVALID_ARG, "conversion workspace too small");
     Carver cv(ws);
     uint64_t *ka = cv.take<uint64_t>(nnz), *kb = cv.take<uint64_t>(nnz);
     uint32_t *pa = cv.take<uint32_t>(nnz), *pb = cv.take<uint32_t>(nnz);

@@ -27,7 +27,9 @@
  * pool (one per device, allocated and freed on the same stream; it keeps at most
  * 256 MB over a synchronization); otherwise pass at
  * least the size the matching *_workspace_size function returns.  A caller
- * workspace must not be used by another call that overlaps on the GPU.
+ * workspace must not be used by another call that overlaps on the GPU.  It starts
+ * on a 16-byte boundary (as every allocation does); one of gsa_coo_to_csr /
+ * gsa_coo_to_csc may start on any byte.
  */
 #ifndef GSA_H
 #define GSA_H
