@@ -1033,17 +1033,16 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
         Rec<VT> *rec1 = (Rec<VT> *)(w + L.rec1);
         VT *val2 = VS ? (VT *)(w + L.val2) : nullptr;
         const bool staged = get_sort_staged() != 0;
-        int sms = 0, optin = 0;
-        if (staged) {
-            int dev = 0;
-            rc = check_cuda(cudaGetDevice(&dev), "bucket: device");
-            if (!rc) rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "bucket: SMs");
-            if (!rc)
-                rc = check_cuda(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev),
-                                "bucket: shared memory");
-            if (rc) return rc;
-        }
-        // dynamic shared memory the staged kernels may take (their static arrays stay below 512 B)
+        int sms = 0, optin = 0, dev = 0;
+        rc = check_cuda(cudaGetDevice(&dev), "bucket: device");
+        if (!rc) rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "bucket: SMs");
+        if (!rc)
+            rc = check_cuda(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev),
+                            "bucket: shared memory");
+        if (rc) return rc;
+        // dynamic shared memory pass C may take (its static arrays stay below 512 B).  Its kernels are
+        // always allowed all of it: the allowance belongs to the function, so one made for a call's own
+        // need could be lowered by another thread before that call's launch.
         const size_t smax = optin > 1024 ? (size_t)optin - 512 : 0;
         // the counting pass: six CTAs of 32 KB histograms per SM, each flushing its counts once
         src.parts([&](const auto &part, int64_t n, int64_t) {
@@ -1075,7 +1074,7 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
         if (fcap >= ST_THREADS) {
             const size_t sm = fine_stage_smem<VT>(co.cs, fcap);
             rc = check_cuda(cudaFuncSetAttribute(fine_stage_kernel<VT, Emit>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax),
                             "bucket: fine_stage_kernel shared memory");
             if (rc) return rc;
             fine_stage_kernel<VT, Emit><<<(unsigned)(co.nb < sms ? co.nb : sms), ST_THREADS, sm, s>>>(
@@ -1085,7 +1084,7 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
         const int stage = stage_entries<VT>(nnz, co.nb);
         const size_t smem = fine_smem_bytes<VT>(co.cs, stage);
         rc = check_cuda(cudaFuncSetAttribute(fine_kernel<VT, Emit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem),
+                                             (int)smax),
                         "bucket: fine_kernel shared memory");
         if (rc) return rc;
         fine_kernel<VT, Emit><<<grid_for(co.nb, 1, 152 * 2), PC_THREADS, smem, s>>>(
