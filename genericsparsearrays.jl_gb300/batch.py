@@ -18,8 +18,8 @@ import torch
 
 from . import _lib
 from .errors import ArgumentError, DimensionMismatch
-from .sparse import (BASE, GenericSparseMatrixCSR, _DTYPE, _ITYPE, _gather_plan, _scalar_buf, _stream_ptr,
-                     nnz)
+from .sparse import (BASE, GenericSparseMatrixCSR, _DTYPE, _ITYPE, _gather_plan, _layout, _scalar_buf,
+                     _stream_ptr, nnz)
 
 ITEM_DTYPE = np.dtype([("rowptr", "<u8"), ("colval", "<u8"), ("nzval", "<u8"), ("B", "<u8"),
                        ("C", "<u8"), ("m", "<i8"), ("n", "<i8"), ("nnz", "<i8"), ("ldb", "<i8"),
@@ -51,19 +51,19 @@ _MODES = {"grouped": _lib.BATCH_GROUPED, "graph": _lib.BATCH_GRAPH, "per_call": 
 
 def _column_major(t: torch.Tensor, what: str) -> Tuple[int, int]:
     """(k, ld) of a vector or column-major matrix operand."""
-    if t.dim() == 1:
-        return 1, max(t.shape[0], 1)
-    if t.dim() == 2 and (t.shape[0] <= 1 or t.stride(0) == 1):
-        ld = t.stride(1) if t.shape[1] > 1 else t.shape[0]
-        return t.shape[1], max(ld, t.shape[0], 1)
+    m = t.unsqueeze(1) if t.dim() == 1 else t
+    if m.dim() == 2:
+        lay, ld = _layout(m)
+        if ld and lay == _lib.OP_N:
+            return m.shape[1], ld
     raise ArgumentError(f"{what} of a grouped product must be a vector or column-major matrix")
 
 
 def _dense_in(t: torch.Tensor) -> Tuple[int, int, int]:
     """(k, ld, rowmajor) of a right-hand side: a vector, a column-major matrix, or a
     row-major one (row i's k values contiguous, rows ld apart)."""
-    if t.dim() == 2 and t.shape[1] > 1 and t.stride(1) == 1 and t.shape[0] > 1:
-        return t.shape[1], max(t.stride(0), t.shape[1]), 1
+    if t.dim() == 2 and t.shape[1] > 1 and t.stride(1) == 1 and t.shape[0] > 1 and t.stride(0) >= t.shape[1]:
+        return t.shape[1], t.stride(0), 1
     if t.dim() == 1 and t.shape[0] > 1 and t.stride(0) != 1:  # a column of a row-major block
         return 1, t.stride(0), 1
     if t.dim() == 2 and t.shape[1] == 1 and t.shape[0] > 1 and t.stride(0) != 1:

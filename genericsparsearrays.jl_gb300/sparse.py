@@ -381,13 +381,27 @@ def _unwrap_sparse(A):
     return A, _lib.OP_N
 
 
+def _layout(t: torch.Tensor) -> Tuple[int, int]:
+    """How the C ABI may read the matrix t where it lies: (OP_N, ld) with element (i, c) at i + c*ld,
+    (OP_T, ld) with it at c + i*ld, ld at least the extent of what is contiguous; ld = 0 where no ld
+    describes t (no unit stride, or columns / rows that share memory)."""
+    r, c = t.shape
+    s0, s1 = t.stride()
+    if (r <= 1 or s0 == 1) and (c <= 1 or (s1 >= r and s1 > 0)):
+        return _lib.OP_N, s1 if c > 1 else max(r, 1)
+    if (c <= 1 or s1 == 1) and (r <= 1 or (s0 >= c and s0 > 0)):
+        return _lib.OP_T, s0 if r > 1 else max(c, 1)
+    return _lib.OP_N, 0
+
+
 def _dense_operand(B) -> Tuple[torch.Tensor, int, int, int, int]:
     """op(B) as (buffer, ldb, opB, rows, cols) for the C ABI.
 
     The C ABI reads op(B)(i, c) = buf[i + c*ld] for opB == N and buf[c + i*ld] (conjugated for
     opB == C) otherwise.  A column-major parent P is used as is; a row-major P is the
     transpose of a column-major buffer, so the op flips.  Only a conjugated row-major parent
-    (op(P) = conj of a column-major buffer) and layouts without a unit stride are copied.
+    (op(P) = conj of a column-major buffer), layouts without a unit stride and views whose
+    columns (rows) share memory, which no ld describes (expand, unfold), are copied.
     """
     op = _lib.OP_N
     if isinstance(B, Adjoint):
@@ -406,19 +420,28 @@ def _dense_operand(B) -> Tuple[torch.Tensor, int, int, int, int]:
         raise ArgumentError("dense operands must be vectors or matrices")
     r, c = t.shape
     rows, cols = (r, c) if op == _lib.OP_N else (c, r)
-    if r <= 1 or t.stride(0) == 1:  # column-major parent
-        ld = t.stride(1) if c > 1 else max(r, 1)
-        return t, max(ld, r, 1), op, rows, cols
-    if c <= 1 or t.stride(1) == 1:  # row-major parent = transpose of a column-major buffer
-        ld = t.stride(0) if r > 1 else max(c, 1)
-        if op == _lib.OP_N:
-            return t, max(ld, c, 1), _lib.OP_T, rows, cols
-        if op == _lib.OP_T:
-            return t, max(ld, c, 1), _lib.OP_N, rows, cols
+    lay, ld = _layout(t)
+    if ld and lay == _lib.OP_N:  # column-major parent
+        return t, ld, op, rows, cols
+    if ld and op != _lib.OP_C:  # row-major parent = transpose of a column-major buffer
+        return t, ld, _lib.OP_T if op == _lib.OP_N else _lib.OP_N, rows, cols
     # copy op(B) into a column-major buffer
     opb = t if op == _lib.OP_N else (t.t() if op == _lib.OP_T else t.conj().t())
     buf = opb.resolve_conj().t().contiguous().t()
     return buf, max(buf.shape[0], 1), _lib.OP_N, rows, cols
+
+
+def _output(C: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, int]:
+    """C as a matrix, the column-major buffer a product writes (C itself, or a copy to be copied
+    back) and its ld.  Columns that share memory hold no result: refused."""
+    C2 = C.unsqueeze(1) if C.dim() == 1 else C
+    r, c = C2.shape
+    lay, ld = _layout(C2)
+    if ld and lay == _lib.OP_N:
+        return C2, C2, ld
+    if (r <= 1 or C2.stride(0) == 1) and C2.numel() > 0:
+        raise ArgumentError("the columns of C must not share memory")
+    return C2, C2.t().contiguous().t(), max(r, 1)
 
 
 def _scalar_buf(v, dtype: torch.dtype):
@@ -539,29 +562,27 @@ def _mul_plain(C, A, B, alpha, beta) -> bool:
         return False
     shape = B.shape
     if len(shape) == 1:
-        r, k = shape[0], 1
-        ldb = r
+        r, k, opB, ldb = shape[0], 1, _lib.OP_N, max(shape[0], 1)
         if r > 1 and B.stride(0) != 1:
             return False
     elif len(shape) == 2:
         r, k = shape
-        if r > 1 and B.stride(0) != 1:
+        opB, ldb = _layout(B)
+        if not ldb or opB != _lib.OP_N:
             return False
-        ldb = B.stride(1) if k > 1 else r
     else:
         return False
     shape = C.shape
     if len(shape) == 1:
-        rc, kc = shape[0], 1
-        ldc = rc
+        rc, kc, opC, ldc = shape[0], 1, _lib.OP_N, max(shape[0], 1)
         if rc > 1 and C.stride(0) != 1:
             return False
     elif len(shape) == 2:
         rc, kc = shape
-        if rc > 1 and C.stride(0) != 1:
-            return False
-        ldc = C.stride(1) if kc > 1 else rc
+        opC, ldc = _layout(C)
     else:
+        return False
+    if not ldc or opC != _lib.OP_N:
         return False
     m, n = P.m, P.n
     if (m, n, k) != ((rc, r, kc) if op == _lib.OP_N else (r, rc, kc)):
@@ -577,7 +598,7 @@ def _mul_plain(C, A, B, alpha, beta) -> bool:
     lib = _lib.load()
     stream = _raw_stream(dev)
     head = (stream, code, icode, m, n, val.numel(), p0.data_ptr(), p1.data_ptr(), val.data_ptr(), BASE, op, k,
-            B.data_ptr(), max(ldb, r, 1), _lib.OP_N, C.data_ptr(), max(ldc, rc, 1), al, be)
+            B.data_ptr(), ldb, _lib.OP_N, C.data_ptr(), ldc, al, be)
     if plan is not None:
         size = lib.gsa_plan_workspace_size(plan.handle, code, k)
         ws = torch.empty(size, dtype=torch.uint8, device=C.device) if size else None
@@ -646,13 +667,7 @@ def mul_(C: torch.Tensor, A, B, alpha=1, beta=0, algo: int = _lib.ALGO_AUTO,
     dev = C.device
     if dev.type != "cuda":
         raise ArgumentError("mul! runs on the GPU only; adapt the operands to CUDA first")
-    # C must be column-major (unit row stride); otherwise compute into a column-major
-    # buffer and copy back.
-    C2 = C.unsqueeze(1) if C.dim() == 1 else C
-    direct = C2.shape[0] <= 1 or C2.stride(0) == 1
-    Cw = C2 if direct else C2.t().contiguous().t()
-    ldc = Cw.stride(1) if Cw.shape[1] > 1 else Cw.shape[0]
-    ldc = max(ldc, Cw.shape[0], 1)
+    C2, Cw, ldc = _output(C)
     lib = _lib.load()
     k = Cc
     stream = _stream_ptr(dev)
@@ -705,7 +720,7 @@ def mul_(C: torch.Tensor, A, B, alpha=1, beta=0, algo: int = _lib.ALGO_AUTO,
                                      al.ctypes.data_as(ctypes.c_void_p),
                                      be.ctypes.data_as(ctypes.c_void_p))
     _lib.check(st)
-    if not direct:
+    if Cw is not C2:
         C2.copy_(Cw)
     return C
 
