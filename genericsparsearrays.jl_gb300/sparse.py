@@ -540,7 +540,7 @@ def _mul_plain(C, A, B, alpha, beta) -> bool:
     op, P = _lib.OP_N, A
     if isinstance(A, Transpose):
         P = A.parent
-        op = _lib.OP_C if type(A) is Adjoint and getattr(P, "dtype", None) in _COMPLEX else _lib.OP_T
+        op = _lib.OP_C if isinstance(A, Adjoint) and getattr(P, "dtype", None) in _COMPLEX else _lib.OP_T
     cls = type(P)
     if cls is GenericSparseMatrixCSR:
         p0, p1 = P.rowptr, P.colval

@@ -119,3 +119,18 @@ def test_products(gsa, cuda, r, c):
                   torch.zeros(m + c - 1, dtype=torch.float64, device=cuda).unfold(0, m, 1).t()):
             with pytest.raises(gsa.ArgumentError):
                 gsa.mul_(C, A, torch.zeros((c, r), dtype=torch.float64, device=cuda).t())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", [torch.float64, torch.complex128])
+def test_subclass_of_adjoint(gsa, cuda, dt):
+    """A wrapper derived from Adjoint is the adjoint in every call, not in the first alone."""
+    class Mine(gsa.Adjoint):
+        pass
+    v = torch.tensor([1 + 2j, 3 - 1j, -2 + 0.5j]).to(dt) if dt.is_complex else torch.tensor([1.0, 3.0, -2.0]).to(dt)
+    A = gsa.adapt(cuda, gsa.GenericSparseMatrixCSR(2, 3, np.array([1, 3, 4]), np.array([1, 3, 2]), v))
+    x = torch.tensor([2.0, -1.0], dtype=dt, device=cuda)
+    want = gsa.mul(gsa.adjoint(A), x)
+    for _ in range(3):
+        y = gsa.mul_(torch.empty(3, dtype=dt, device=cuda), Mine(A), x)
+        assert torch.equal(y, want)
