@@ -94,6 +94,19 @@ cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s) {
     return cudaMallocAsync(p, bytes, s);
 }
 
+// Waits for all work of the current device, on whatever stream.  cudaDeviceSynchronize is not allowed
+// while a stream of the device is being captured, and ends that capture, also when the capture is
+// another thread's or a relaxed one (a batch captures its launch in one thread while another drops a
+// matrix); freeing an allocation of cudaMalloc waits as well, and is allowed then.
+static int device_wait(const char *what) {
+    void *token = nullptr;
+    if (cudaMalloc(&token, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return check_cuda(cudaDeviceSynchronize(), what);
+    }
+    return check_cuda(cudaFree(token), what);
+}
+
 // A stream per device that only memory is given back on, ordered after an event of its last use.
 static std::atomic<cudaStream_t> g_free_streams[POOL_DEVICES];
 
@@ -124,9 +137,9 @@ int scratch_free_after(int device, cudaEvent_t used, std::initializer_list<void 
         fs = nullptr;
     }
     int rc = GSA_OK;
-    if (!fs) rc = check_cuda(cudaDeviceSynchronize(), "free: sync");
+    if (!fs) rc = device_wait("free: sync");
     for (void *p : mem) {
-        if (!p) continue;
+        if (!p || (!fs && rc)) continue;  // work may still use what could not be waited for
         const int rc2 = check_cuda(fs ? cudaFreeAsync(p, fs) : cudaFree(p), "free");
         if (!rc) rc = rc2;
     }
@@ -135,16 +148,15 @@ int scratch_free_after(int device, cudaEvent_t used, std::initializer_list<void 
 }
 
 // Frees a plan's device memory.  Work on any stream may still read it, so the plan's device is
-// synchronized first (as cudaFree of a cudaMalloc allocation does by itself).
+// waited for first; if that fails the memory stays.
 static int plan_release(Plan *p) {
     int rc = GSA_OK, dev = 0;
     if (p->mem || p->coo_ptr) {
         const bool moved = cudaGetDevice(&dev) == cudaSuccess && dev != p->device;
         if (moved) cudaSetDevice(p->device);
-        rc = check_cuda(cudaDeviceSynchronize(), "plan: free");
-        if (p->coo_ptr) cudaFree(p->coo_ptr);
+        rc = device_wait("plan: free");
+        if (p->coo_ptr && !rc) rc = check_cuda(cudaFree(p->coo_ptr), "plan: free");
         if (p->mem && !rc) rc = check_cuda(cudaFree(p->mem), "plan: free");
-        else if (p->mem) cudaFree(p->mem);
         if (moved) cudaSetDevice(dev);
     }
     delete p;

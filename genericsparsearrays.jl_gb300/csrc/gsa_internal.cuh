@@ -379,7 +379,7 @@ int radix_bits_for(int64_t count);  // bits that values 0 .. count - 1 need
 // the device has been synchronized (cudaFree waits for nothing on such memory).
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s);
 // Gives memory of scratch_alloc back once `used` has passed, without waiting for it here (NULL:
-// the device is synchronized instead).
+// the device is waited for instead).
 int scratch_free_after(int device, cudaEvent_t used, std::initializer_list<void *> mem);
 
 // Scratch of one call: the caller's buffer, or a stream-ordered allocation freed on the

@@ -922,8 +922,8 @@ struct SpgemmComputeBody {
 
 // After work of the handle on stream s: `used` covers it while all of it is on one stream and runs
 // now.  Work on a second stream and captured work (its graph runs when the program says) are
-// covered by no one event, and what cannot be told or recorded by none: the handle's memory then
-// goes through a synchronization of the device.
+// covered by no one event, and what cannot be told or recorded by none: the handle's memory is then
+// given back after a wait for the device.
 static void spgemm_used(gsa_spgemm *h, cudaStream_t s) {
     std::lock_guard<std::mutex> hold(h->lock);
     if (h->many) return;
