@@ -14,6 +14,7 @@
 // power-law lengths and 20 to 40 ms for the 4.2M rows of the 2048^2 grid -- hundreds of products
 // of the matrix -- before the first product of every new matrix.
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "gsa_rows.cuh"
@@ -300,23 +301,41 @@ bin_order_kernel(int64_t outer_n, int64_t nnz, const I *__restrict__ ptr, int ba
     }
 }
 
-// Host memory that a kernel writes its few counts to: one page per host thread, which waits for
-// the kernel before it reads, and given back when the thread ends.  NULL where it cannot be had.
+// Host memory that a kernel writes its few counts to: a page that a call has to itself, taken from
+// and returned to a list of the process (no page is freed when a thread ends: that is not allowed
+// while another thread captures a stream, and would end its capture).  At most MAX_BOXES pages exist;
+// p is NULL where none can be had.
 constexpr size_t COUNT_BOX = 4096;
-char *count_box() {
-    struct Box {
-        void *p = nullptr;
-        ~Box() {
-            if (p) cudaFreeHost(p);
+constexpr int MAX_BOXES = 64;
+std::mutex g_boxes_lock;
+char *g_boxes[MAX_BOXES];
+int g_boxes_free = 0, g_boxes_made = 0;
+struct CountBox {
+    char *p = nullptr;
+    bool take() {
+        std::unique_lock<std::mutex> hold(g_boxes_lock);
+        if (g_boxes_free > 0) {
+            p = g_boxes[--g_boxes_free];
+        } else if (g_boxes_made < MAX_BOXES) {
+            ++g_boxes_made;
+            hold.unlock();
+            void *q = nullptr;
+            if (cudaHostAlloc(&q, COUNT_BOX, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+                p = (char *)q;
+            } else {
+                cudaGetLastError();
+                hold.lock();
+                --g_boxes_made;
+            }
         }
-    };
-    static thread_local Box box;
-    if (!box.p && cudaHostAlloc(&box.p, COUNT_BOX, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-        cudaGetLastError();
-        box.p = nullptr;
+        return p != nullptr;
     }
-    return (char *)box.p;
-}
+    ~CountBox() {
+        if (!p) return;
+        std::lock_guard<std::mutex> hold(g_boxes_lock);
+        g_boxes[g_boxes_free++] = p;
+    }
+};
 
 template <typename I>
 int build_plan(cudaStream_t s, int64_t outer_n, int64_t nnz, const I *ptr, int base, Plan *p) {
@@ -335,15 +354,17 @@ int build_plan(cudaStream_t s, int64_t outer_n, int64_t nnz, const I *ptr, int b
     const size_t o_cnt = sc.reserve<PlanCount>((size_t)nct);
     const size_t bytes1 = sc.off;
     std::vector<char> copied;
+    CountBox box;
     const char *got = nullptr;
     auto count = [&](char *d) {
         plan_stats_kernel<I><<<(unsigned)nct, PL_THREADS, 0, s>>>(outer_n, nnz, ptr, base, rows, (PlanTotals *)(d + o_tot),
                                                                   (PlanCount *)(d + o_cnt), (uint32_t *)(d + o_hist));
         return check_cuda(cudaGetLastError(), "plan_stats_kernel");
     };
-    if (nct == 1 && bytes1 <= COUNT_BOX && (got = count_box())) {
+    if (nct == 1 && bytes1 <= COUNT_BOX && box.take()) {
         // one CTA: its sums go straight to host memory, without scratch and a copy (30 us a plan with)
-        int rc = count((char *)got);
+        got = box.p;
+        int rc = count(box.p);
         if (!rc) rc = check_cuda(cudaStreamSynchronize(s), "plan: sync");
         if (rc) return rc;
     } else {

@@ -73,6 +73,30 @@ def test_dropped_during_a_capture(gsa, cuda, what, mode, other):
     assert torch.equal(y, want)
 
 
+def test_planning_thread_ends_during_a_capture(gsa, cuda):
+    A, x, want = matrix(gsa, cuda, 3000, 700)
+    go, planned = threading.Event(), threading.Event()
+    kept = []
+
+    def work():
+        kept.append(matrix(gsa, cuda, 300, 40))
+        torch.cuda.synchronize()
+        planned.set()
+        go.wait()
+    t = threading.Thread(target=work)
+    t.start()
+    planned.wait()
+    y = torch.zeros_like(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="global"):
+        gsa.mul_(y, A, x)
+        go.set()
+        t.join()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+
+
 @pytest.mark.parametrize("what", ["plan", "spgemm"])
 def test_dropping_waits_for_every_stream(gsa, cuda, what):
     """No event tells what reads a plan or a handle of several streams: all work has finished."""
@@ -90,3 +114,24 @@ def test_dropping_waits_for_every_stream(gsa, cuda, what):
     else:
         M.__dict__.pop("_plan")
     assert done.query()
+
+
+def test_threads_that_plan_at_once(gsa, cuda):
+    """Small plans of many threads, each with its counts to itself."""
+    wrong = []
+
+    def work(seed):
+        rng = np.random.default_rng(seed)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for n, long in ((200, 40), (2000, 600), (300, 290)):
+                for _ in range(10):
+                    A, x, y = matrix(gsa, cuda, n, long, int(rng.integers(1 << 30)))
+                    torch.cuda.current_stream().synchronize()
+                    if A._plan is None or A._plan.max_len != long:
+                        wrong.append((seed, n))
+    threads = [threading.Thread(target=work, args=(s,)) for s in range(12)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
