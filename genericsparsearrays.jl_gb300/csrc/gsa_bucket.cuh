@@ -20,7 +20,7 @@
 //      memory (cs is chosen so that an average bucket fills at most half of the staging).  Every
 //      entry of a row of up to 256 counts the row's smaller keys and writes itself to its place.
 //      Longer rows go to the kernels of longer rows: chunks of 4096 entries sorted by a CTA each,
-//      then merged by counting (values gathered by input position).  A bucket larger than the
+//      then merged by counting, in groups (values gathered by input position).  A bucket larger than the
 //      staging is placed in global memory instead, its rows of up to 16 entries sorted by a
 //      thread, up to 256 by a warp (warp_kernel).  Where rows average at most 8 entries,
 //      fine_stage_kernel runs this pass instead: one CTA per SM, the next bucket's records copied
@@ -43,6 +43,7 @@
 #pragma once
 
 #include <type_traits>
+#include <utility>
 
 #include "gsa_internal.cuh"
 
@@ -53,6 +54,9 @@ constexpr int SMALL = 16;          // a thread sorts rows of up to 16 entries in
 constexpr int WARP_MAX = 256;      // a warp sorts rows of up to 256 entries
 constexpr int LONG_THREADS = 512;
 constexpr int LONG_CHUNK = 4096;   // entries of a longer row that a CTA sorts in shared memory (32 KB)
+constexpr int64_t LONG_ONE_PASS = (int64_t)1 << 24;  // entries of a sort whose longer rows are merged in one pass
+constexpr int LONG_FAN = 64;       // else: chunks merged together in the first pass,
+constexpr int MERGE_FAN = 256;     // and the runs that this leaves in each further one
 constexpr int WARP_CTA_THREADS = 256;
 constexpr int ROWS_MAX = 4096;     // rows per coarse bucket
 constexpr int COARSE_MAX = 8192;   // coarse buckets, the invalid-row bucket included
@@ -181,7 +185,8 @@ inline Layout layout(int64_t major_n, int64_t minor_n, int64_t nnz, size_t vsize
     L.start = cv.reserve<uint32_t>(major_n + 2);
     L.bsums = cv.reserve<uint32_t>(ceil_div(nscan, (int64_t)sc_tile) + 1);
     L.key1 = L.co.ok ? 0 : cv.reserve<uint64_t>(n);
-    L.key2 = L.co.ok ? cv.reserve<uint64_t>(n) : 0;
+    // (the one-level form's second buffer for the further passes over long rows)
+    L.key2 = L.co.ok || n > LONG_ONE_PASS ? cv.reserve<uint64_t>(n) : 0;
     L.rec1 = L.co.ok ? cv.reserve<unsigned char>((size_t)n * rec_size(vsize)) : 0;
     L.val2 = L.co.ok && vsize ? cv.reserve<unsigned char>((size_t)n * vsize) : 0;
     L.list = cv.reserve<uint32_t>(major_n + 1);
@@ -896,7 +901,7 @@ __device__ __forceinline__ void bitonic_shared(uint64_t *s, uint32_t P) {
     }
 }
 
-// Rows of more than WARP_MAX entries, in two kernels, a CTA per listed chunk of LONG_CHUNK entries.
+// Rows of more than WARP_MAX entries, a CTA per listed chunk of LONG_CHUNK entries.
 // long_sort_kernel sorts a chunk in shared memory and writes the row if that is all of it;
 // long_merge_kernel gives every entry of a row of several chunks its place: its own in its chunk
 // plus, for each other chunk (read into shared memory in turn), the number of smaller keys there.
@@ -904,9 +909,14 @@ __device__ __forceinline__ void bitonic_shared(uint64_t *s, uint32_t P) {
 //
 // A row's chunks are spread over the SMs, so the longest row sets no tail: one CTA per row, chunk
 // sorts, pairwise merges and all, took 1.0 to 1.2 ms for the power-law matrix of 10^6 rows, one SM
-// busy with its row of 50,000 entries all that time, against 0.12 (sort) and 0.07 ms
-// (merge).  The work of a row grows with the square of
-// its chunks, and stays below the pairwise merges' up to rows of some 10^8 entries.
+// busy with its row of 50,000 entries all that time, against 0.12 (sort) and 0.07 ms (merge).
+//
+// One such pass costs a row the square of its chunks: a row of 10^6 entries 1.4 ms, of 3*10^7 1.1 s,
+// of 10^8 11.9 s.  Sorts of more than LONG_ONE_PASS entries therefore merge in groups: of LONG_FAN
+// chunks first, then of MERGE_FAN of the runs that the pass before left, until a row is one run
+// (merge_runs_kernel).  An entry is then searched in at most LONG_FAN + MERGE_FAN places per pass,
+// whatever the row's length.  Fewer entries than that make one pass do: each further one is a launch
+// (2 us) that nearly every matrix has no row for.
 template <class Emit>
 __global__ void __launch_bounds__(LONG_THREADS)
 long_sort_kernel(const uint32_t *__restrict__ start, uint64_t *keys, LongRows longs, Emit emit) {
@@ -932,9 +942,29 @@ long_sort_kernel(const uint32_t *__restrict__ start, uint64_t *keys, LongRows lo
     }
 }
 
+// The keys of s[0 .. m) that are smaller than each of a thread's keys, added to rank: all keys one
+// step at a time.
+template <int PER>
+__device__ __forceinline__ void count_smaller(const uint64_t *s, uint32_t m, const uint64_t (&k)[PER],
+                                              uint32_t (&rank)[PER]) {
+    uint32_t at[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) at[u] = 0;
+    for (uint32_t step = LONG_CHUNK; step > 0; step >>= 1) {
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+            if (at[u] + step <= m && s[at[u] + step - 1] < k[u]) at[u] += step;
+    }
+#pragma unroll
+    for (int u = 0; u < PER; ++u) rank[u] += at[u];
+}
+
+// Merges the chunks of a row in groups of `fan`: rows of one group are written, others left as runs of
+// fan chunks in `out`.
 template <class Emit>
 __global__ void __launch_bounds__(LONG_THREADS)
-long_merge_kernel(const uint32_t *__restrict__ start, const uint64_t *__restrict__ keys, LongRows longs, Emit emit) {
+long_merge_kernel(const uint32_t *__restrict__ start, const uint64_t *__restrict__ keys, uint64_t *__restrict__ out,
+                  uint32_t fan, LongRows longs, Emit emit) {
     __shared__ uint64_t s[LONG_CHUNK];
     constexpr int PER = LONG_CHUNK / LONG_THREADS;
     const uint32_t nitems = longs.counters[1];
@@ -943,15 +973,16 @@ long_merge_kernel(const uint32_t *__restrict__ start, const uint64_t *__restrict
         const uint32_t b = start[item.x], len = start[item.x + 1] - b, c0 = item.y * LONG_CHUNK;
         if (len <= (uint32_t)LONG_CHUNK) continue;  // the whole CTA
         const uint32_t n = len - c0 < (uint32_t)LONG_CHUNK ? len - c0 : (uint32_t)LONG_CHUNK;
+        const uint32_t nchunks = (len - 1) / LONG_CHUNK + 1;
+        const uint32_t d0 = item.y / fan * fan, d1 = nchunks - d0 < fan ? nchunks : d0 + fan;  // the group
         uint64_t k[PER];
         uint32_t rank[PER];
 #pragma unroll
         for (int u = 0; u < PER; ++u) {
             const uint32_t j = (uint32_t)(u * LONG_THREADS) + threadIdx.x;
             k[u] = j < n ? keys[b + c0 + j] : 0ull;
-            rank[u] = j;
+            rank[u] = d0 * LONG_CHUNK + j;
         }
-        const uint32_t nchunks = (len - 1) / LONG_CHUNK + 1;
         auto size_of = [&](uint32_t d) {
             const uint32_t left = len - d * LONG_CHUNK;
             return left < (uint32_t)LONG_CHUNK ? left : (uint32_t)LONG_CHUNK;
@@ -965,41 +996,121 @@ long_merge_kernel(const uint32_t *__restrict__ start, const uint64_t *__restrict
                 ahead[u] = j < m ? keys[b + d * LONG_CHUNK + j] : ~0ull;
             }
         };
-        uint32_t d = item.y == 0 ? 1u : 0u;
-        read(d);  // the row has another chunk
-        while (d < nchunks) {
+        uint32_t d = item.y == d0 ? d0 + 1 : d0;
+        if (d < d1) read(d);
+        while (d < d1) {
             const uint32_t m = size_of(d);
 #pragma unroll
             for (int u = 0; u < PER; ++u) s[u * LONG_THREADS + threadIdx.x] = ahead[u];
             __syncthreads();
             d += d + 1 == item.y ? 2u : 1u;
-            if (d < nchunks) read(d);
-            // smaller keys of the chunk, all of a thread's keys one step at a time
-            uint32_t at[PER];
-#pragma unroll
-            for (int u = 0; u < PER; ++u) at[u] = 0;
-            for (uint32_t step = LONG_CHUNK; step > 0; step >>= 1) {
-#pragma unroll
-                for (int u = 0; u < PER; ++u)
-                    if (at[u] + step <= m && s[at[u] + step - 1] < k[u]) at[u] += step;
-            }
-#pragma unroll
-            for (int u = 0; u < PER; ++u) rank[u] += at[u];
+            if (d < d1) read(d);
+            count_smaller<PER>(s, m, k, rank);
             __syncthreads();
         }
 #pragma unroll
         for (int u = 0; u < PER; ++u)
-            if ((uint32_t)(u * LONG_THREADS) + threadIdx.x < n) emit.gather(b + rank[u], (uint64_t)item.x, k[u]);
+            if ((uint32_t)(u * LONG_THREADS) + threadIdx.x < n) {
+                if (nchunks <= fan) emit.gather(b + rank[u], (uint64_t)item.x, k[u]);
+                else out[b + rank[u]] = k[u];
+            }
     }
 }
 
-// The rows that the passes before left, keys in row order in `keys` (and values in `vals`).
+// The keys of p[0 .. n), sorted, that are smaller than x.
+__device__ __forceinline__ uint32_t lower_bound(const uint64_t *p, uint32_t n, uint64_t x) {
+    uint32_t lo = 0;
+    while (n > 0) {
+        const uint32_t half = n >> 1;
+        const bool less = p[lo + half] < x;
+        lo = less ? lo + half + 1 : lo;
+        n = less ? n - half - 1 : half;
+    }
+    return lo;
+}
+
+// A further pass over rows longer than `run`, which are runs of that many sorted entries: groups of
+// MERGE_FAN runs become one run in `out`, or are written where that is the whole row.  A CTA places a
+// chunk's entries: in each other run of the group only those between the chunk's first and last key
+// are searched (a thread per run finds them), the ones before are all smaller.  Over a run's chunks
+// these stretches make up the other runs once, so the work per entry does not grow with the row.
+template <class Emit>
+__global__ void __launch_bounds__(LONG_THREADS)
+merge_runs_kernel(const uint32_t *__restrict__ start, const uint64_t *__restrict__ keys, uint64_t *__restrict__ out,
+                  uint32_t run, LongRows longs, Emit emit) {
+    static_assert(MERGE_FAN <= LONG_THREADS, "a thread per run");
+    __shared__ uint64_t s[LONG_CHUNK];
+    __shared__ uint32_t s_lo[MERGE_FAN], s_hi[MERGE_FAN];
+    constexpr int PER = LONG_CHUNK / LONG_THREADS;
+    const uint32_t nitems = longs.counters[1];
+    const uint64_t group = (uint64_t)run * MERGE_FAN;
+    for (uint32_t q = blockIdx.x; q < nitems; q += gridDim.x) {
+        const uint2 item = longs.items[q];
+        const uint32_t b = start[item.x], len = start[item.x + 1] - b, c0 = item.y * LONG_CHUNK;
+        if (len <= run) continue;  // the whole CTA: written by a pass before
+        const uint32_t n = len - c0 < (uint32_t)LONG_CHUNK ? len - c0 : (uint32_t)LONG_CHUNK;
+        const uint32_t g0 = (uint32_t)(c0 / group * group), glen = len - g0 < group ? len - g0 : (uint32_t)group;
+        const uint32_t own = (c0 - g0) / run, nruns = (glen - 1) / run + 1;
+        const uint64_t *gk = keys + b + g0;
+        uint64_t k[PER];
+        uint32_t rank[PER];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const uint32_t j = (uint32_t)(u * LONG_THREADS) + threadIdx.x;
+            k[u] = j < n ? keys[b + c0 + j] : 0ull;
+            rank[u] = c0 - g0 - own * run + j;
+        }
+        if (threadIdx.x < nruns && threadIdx.x != own) {
+            const uint64_t *p = gk + threadIdx.x * run;
+            const uint32_t left = glen - threadIdx.x * run, m = left < run ? left : run;
+            const uint32_t lo = lower_bound(p, m, keys[b + c0]);
+            s_lo[threadIdx.x] = lo;
+            s_hi[threadIdx.x] = lo + lower_bound(p + lo, m - lo, keys[b + c0 + n - 1]);
+        }
+        __syncthreads();
+        for (uint32_t d = 0; d < nruns; ++d) {
+            if (d == own) continue;
+            const uint32_t hi = s_hi[d];
+            const uint64_t *p = gk + d * run;
+#pragma unroll
+            for (int u = 0; u < PER; ++u) rank[u] += s_lo[d];
+            for (uint32_t t = s_lo[d]; t < hi;) {
+                const uint32_t m = hi - t < (uint32_t)LONG_CHUNK ? hi - t : (uint32_t)LONG_CHUNK;
+#pragma unroll
+                for (int u = 0; u < PER; ++u) {
+                    const uint32_t j = (uint32_t)(u * LONG_THREADS) + threadIdx.x;
+                    if (j < m) s[j] = p[t + j];
+                }
+                __syncthreads();
+                count_smaller<PER>(s, m, k, rank);
+                __syncthreads();
+                t += m;
+            }
+        }
+        __syncthreads();  // s_lo and s_hi have been read
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+            if ((uint32_t)(u * LONG_THREADS) + threadIdx.x < n) {
+                if (len <= group) emit.gather(b + rank[u], (uint64_t)item.x, k[u]);
+                else out[b + g0 + rank[u]] = k[u];
+            }
+    }
+}
+
+// The rows that the passes before left, keys in row order in `keys` (and values in `vals`); `other`
+// holds as many keys (used by sorts of more than LONG_ONE_PASS entries).
 template <class VT, class Emit>
-int launch_long_rows(cudaStream_t s, const uint32_t *start, uint64_t *keys, const VT *vals, const LongRows &longs,
-                     const Emit &emit) {
+int launch_long_rows(cudaStream_t s, int64_t nnz, const uint32_t *start, uint64_t *keys, uint64_t *other, const VT *vals,
+                     const LongRows &longs, const Emit &emit) {
+    const bool once = nnz <= LONG_ONE_PASS;
     warp_kernel<VT, Emit><<<152 * 8, WARP_CTA_THREADS, 0, s>>>(start, keys, vals, longs, emit);
     long_sort_kernel<Emit><<<152 * 4, LONG_THREADS, 0, s>>>(start, keys, longs, emit);
-    long_merge_kernel<Emit><<<152 * 4, LONG_THREADS, 0, s>>>(start, keys, longs, emit);
+    long_merge_kernel<Emit><<<152 * 4, LONG_THREADS, 0, s>>>(start, keys, other, once ? 0xffffffffu : (uint32_t)LONG_FAN,
+                                                             longs, emit);
+    for (int64_t run = (int64_t)LONG_CHUNK * LONG_FAN; !once && run < nnz; run *= MERGE_FAN) {
+        merge_runs_kernel<Emit><<<152 * 4, LONG_THREADS, 0, s>>>(start, other, keys, (uint32_t)run, longs, emit);
+        std::swap(keys, other);
+    }
     return check_cuda(cudaGetLastError(), "bucket sort kernels");
 }
 
@@ -1079,7 +1190,7 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
             if (rc) return rc;
             fine_stage_kernel<VT, Emit><<<(unsigned)(co.nb < sms ? co.nb : sms), ST_THREADS, sm, s>>>(
                 major_n, co, fcap, cstart, rec1, key2, val2, start, longs, emit);
-            return launch_long_rows<VT, Emit>(s, start, key2, val2, longs, emit);
+            return launch_long_rows<VT, Emit>(s, nnz, start, key2, (uint64_t *)rec1, val2, longs, emit);
         }
         const int stage = stage_entries<VT>(nnz, co.nb);
         const size_t smem = fine_smem_bytes<VT>(co.cs, stage);
@@ -1089,7 +1200,7 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
         if (rc) return rc;
         fine_kernel<VT, Emit><<<grid_for(co.nb, 1, 152 * 2), PC_THREADS, smem, s>>>(
             major_n, co, stage, cstart, rec1, key2, val2, start, longs, emit);
-        return launch_long_rows<VT, Emit>(s, start, key2, val2, longs, emit);
+        return launch_long_rows<VT, Emit>(s, nnz, start, key2, (uint64_t *)rec1, val2, longs, emit);
     }
     src.parts([&](const auto &part, int64_t n, int64_t) {
         using P = std::decay_t<decltype(part)>;
@@ -1104,7 +1215,7 @@ int sort(cudaStream_t s, int64_t major_n, int64_t minor_n, int64_t nnz, const Sr
         if (n > 0) place_kernel<P><<<grid_for(n, 256, cap), 256, 0, s>>>(part, n, first, major_n, start, cnt, key1);
     });
     small_kernel<Emit><<<grid_for(major_n + 1, 256, 152 * 32), 256, 0, s>>>(major_n, start, key1, longs, emit);
-    return launch_long_rows<NoValue, Emit>(s, start, key1, nullptr, longs, emit);
+    return launch_long_rows<NoValue, Emit>(s, nnz, start, key1, key2, nullptr, longs, emit);
 }
 
 }  // namespace bucket
