@@ -315,21 +315,27 @@ merge_rows_kernel(int64_t outer_n, const uint32_t *__restrict__ merged, const I 
             for (int c = 1; c < K; ++c) jmin = jc[c] < jmin ? jc[c] : jmin;
             if (left == 0) jmin = END;
             if (!__any_sync(0xffffffffu, jmin != END)) break;
-            if (jmin != END) {
-                V acc = VT<V>::zero();
-                bool first = true;
+            const bool live = jmin != END;
+            V acc = VT<V>::zero();
+            bool first = true;
 #pragma unroll
-                for (int c = 0; c < K; ++c) {
-                    while (jc[c] == jmin) {
+            for (int c = 0; c < K; ++c) {
+                bool hit = live && jc[c] == jmin;
+                while (__any_sync(0xffffffffu, hit)) {  // the whole warp: again for a repeated column
+                    // 0 + x without the FP64 add, where no lane needs one
+                    const bool adds = __any_sync(0xffffffffu, hit && !first);
+                    if (hit) {
                         const V x = product(a[c], ldg(qv + cur[c]), csr);
-                        // 0 + x without the FP64 add, where no lane needs one
-                        if (__any_sync(__activemask(), !first)) acc = first ? zero_plus(x) : add(acc, x);
+                        if (adds) acc = first ? zero_plus(x) : add(acc, x);
                         else acc = zero_plus(x);
                         first = false;
                         ++cur[c];
                         jc[c] = cur[c] < end[c] ? (uint32_t)__ldg(qi + cur[c]) - (uint32_t)base : END;
+                        hit = jc[c] == jmin;
                     }
                 }
+            }
+            if (live) {
                 s_j[w][held * LD + lane] = jmin;
                 s_v[w][held * LD + lane] = acc;
                 ++held;
