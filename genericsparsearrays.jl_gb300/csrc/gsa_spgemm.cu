@@ -347,7 +347,8 @@ merge_rows_kernel(int64_t outer_n, const uint32_t *__restrict__ merged, const I 
     write_held();
 }
 
-// Thread per listed tiny row (at most SG_TINY_P products): the same expansion, sums and
+// Thread per listed tiny row (at most SG_TINY_P products; the rows that count_rows_kernel could not
+// merge: more than SG_TINY_A entries, or a Q row that is not sorted): the same expansion, sums and
 // positions as small_kernel, each thread in its own column of the warp's shared block
 // (slot s of lane l at s * 32 + l, so the lanes never share a bank), the first products of
 // each column kept as a bit mask.
@@ -398,50 +399,6 @@ tiny_kernel(const uint32_t *__restrict__ list, const uint32_t *__restrict__ coun
 #pragma unroll
             for (int c = 0; c < SG_TINY_A; ++c)
                 if (len[c]) expand(qb[c], len[c], NUMERIC ? a[c] : V{});
-            // The products are SG_TINY_A runs, one per A entry, in A order.  When every run is
-            // sorted by column (sorted Q rows), a merge of the runs visits the columns in
-            // increasing order and, for each, its products in the reference's order (runs in A
-            // order, each run in its own order): no quadratic scan.
-            uint32_t hs[SG_TINY_A], he[SG_TINY_A];
-            uint32_t off = 0;
-            bool sorted = true;
-#pragma unroll
-            for (int c = 0; c < SG_TINY_A; ++c) {
-                hs[c] = off < P ? off : P;
-                off += len[c];
-                he[c] = off < P ? off : P;
-                for (uint32_t u = hs[c] + 1; u < he[c]; ++u)
-                    if (tj[w][u * 32 + lane] < tj[w][(u - 1) * 32 + lane]) sorted = false;
-            }
-            if (sorted) {
-                uint64_t jc[SG_TINY_A];
-#pragma unroll
-                for (int c = 0; c < SG_TINY_A; ++c) jc[c] = hs[c] < he[c] ? tj[w][hs[c] * 32 + lane] : ~0ull;
-                const uint32_t out0 = NUMERIC ? cptr[o] : 0;
-                uint32_t count = 0;
-                for (uint32_t guard = 0; guard <= (uint32_t)SG_TINY_P; ++guard) {
-                    uint64_t jmin = jc[0];
-#pragma unroll
-                    for (int c = 1; c < SG_TINY_A; ++c) jmin = jc[c] < jmin ? jc[c] : jmin;
-                    if (jmin == ~0ull) break;
-                    V acc = VT<V>::zero();
-#pragma unroll
-                    for (int c = 0; c < SG_TINY_A; ++c) {
-                        while (jc[c] == jmin) {
-                            if constexpr (NUMERIC) acc = add(acc, tv[w][hs[c] * 32 + lane]);
-                            ++hs[c];
-                            jc[c] = hs[c] < he[c] ? tj[w][hs[c] * 32 + lane] : ~0ull;
-                        }
-                    }
-                    if constexpr (NUMERIC) {
-                        idx_out[out0 + count] = (I)((int64_t)jmin + base);
-                        val_out[out0 + count] = acc;
-                    }
-                    ++count;
-                }
-                if constexpr (!NUMERIC) cnt[o] = count;
-                continue;
-            }
         } else {
             for (int64_t t = b; t < e; ++t) {
                 const int64_t k = (int64_t)__ldg(pi + t) - base;
