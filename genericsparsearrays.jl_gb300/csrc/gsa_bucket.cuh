@@ -21,7 +21,7 @@
 //      entry of a row of up to 256 counts the row's smaller keys and writes itself to its place.
 //      Longer rows go to the kernels of longer rows: chunks of 4096 entries sorted by a CTA each,
 //      then merged by counting, in groups (values gathered by input position).  A bucket larger than the
-//      staging is placed in global memory instead, its rows of up to 16 entries sorted by a
+//      staging is placed in global memory instead, its rows of up to 8 entries sorted by a
 //      thread, up to 256 by a warp (warp_kernel).  Where rows average at most 8 entries,
 //      fine_stage_kernel runs this pass instead: one CTA per SM, the next bucket's records copied
 //      into shared memory while the current one is sorted, the bucket's output written with
@@ -50,7 +50,13 @@
 namespace gsa {
 namespace bucket {
 
-constexpr int SMALL = 16;          // a thread sorts rows of up to 16 entries in registers
+// A thread sorts rows of up to 8 entries in registers; in small_kernel, whose registers are not
+// bounded, of up to 16.  (In the kernels of pass C, held to 64 registers, a thread's sort of 16 keys
+// runs partly from spilled registers.  In two of them -- the in-place sort of fine_stage_kernel and the
+// emitting one of a fine_kernel without values -- it went wrong on GB300, though its logic is right
+// on the CPU: rows unsorted, places unwritten, then reads through what the places held.)
+constexpr int SMALL = 8;
+constexpr int SMALL_UNBOUNDED = 16;
 constexpr int WARP_MAX = 256;      // a warp sorts rows of up to 256 entries
 constexpr int LONG_THREADS = 512;
 constexpr int LONG_CHUNK = 4096;   // entries of a longer row that a CTA sorts in shared memory (32 KB)
@@ -232,15 +238,16 @@ __device__ __forceinline__ void sort_registers(const uint64_t *keys, const VT *v
     }
 }
 
-template <class Emit, class VT>
+// Rows of up to MOST entries (8 or 16).
+template <int MOST, class Emit, class VT>
 __device__ __forceinline__ void sort_short_row(const uint64_t *keys, const VT *vals, uint32_t out, uint32_t len,
                                                uint64_t r, const Emit &emit) {
     if (len <= 4) sort_registers<Emit, VT, 4>(keys, vals, out, len, r, emit);
     else if (len <= 8) sort_registers<Emit, VT, 8>(keys, vals, out, len, r, emit);
-    else if (len <= SMALL) sort_registers<Emit, VT, SMALL>(keys, vals, out, len, r, emit);
+    else if (MOST > 8 && len <= MOST) sort_registers<Emit, VT, MOST>(keys, vals, out, len, r, emit);
 }
 
-// What is left for the kernels of longer rows: rows of (SMALL, WARP_MAX] entries (list, counted
+// What is left for the kernels of longer rows: rows of (SHORT, WARP_MAX] entries (list, counted
 // in counters[0]) and the chunks of LONG_CHUNK entries of still longer ones (items: row, chunk;
 // counters[1]).
 struct LongRows {
@@ -249,8 +256,9 @@ struct LongRows {
     uint32_t *counters;
 };
 // One atomic per warp and kind.  All 32 lanes call this.
+template <int SHORT>
 __device__ __forceinline__ void list_long_rows(bool valid, uint32_t len, uint32_t r, const LongRows &L) {
-    const bool to_warp = valid && len > SMALL && len <= WARP_MAX;
+    const bool to_warp = valid && len > SHORT && len <= WARP_MAX;
     const bool to_items = valid && len > WARP_MAX;
     const unsigned mw = __ballot_sync(0xffffffffu, to_warp), mi = __ballot_sync(0xffffffffu, to_items);
     const int lane = threadIdx.x & 31;
@@ -385,7 +393,7 @@ template <class VT> inline size_t fine_smem_bytes(int cs, int stage) {
 // CTA per coarse bucket, taken from a queue (counters[2]): rows counted and scanned in shared
 // memory (the row pointers), then the bucket's keys placed in row order -- into shared memory when
 // the bucket fits the staging, else into key2 / val2 (read back in this kernel: plain pointers, no
-// read-only cache path) with rows of more than 16 entries listed for the kernels of longer rows.
+// read-only cache path) with rows of more than 8 entries listed for the kernels of longer rows.
 //
 // Staged, every entry of a row of up to 256 finds its place by counting the row's smaller keys, a
 // thread per entry whatever its row: consecutive threads hold the entries of a row, so their reads
@@ -498,7 +506,7 @@ fine_kernel(int64_t major_n, Coarse co, int stage, const uint32_t *__restrict__ 
                 for (int j0 = 0; j0 < R; j0 += PC_THREADS) {
                     const int j = j0 + threadIdx.x;
                     const uint32_t len = j < R ? s_off[j + 1] - s_off[j] : 0u;
-                    list_long_rows(len > (uint32_t)WARP_MAX, len, (uint32_t)(row0 + j), longs);
+                    list_long_rows<WARP_MAX>(len > (uint32_t)WARP_MAX, len, (uint32_t)(row0 + j), longs);
                 }
             }
         } else {
@@ -517,9 +525,9 @@ fine_kernel(int64_t major_n, Coarse co, int stage, const uint32_t *__restrict__ 
                     const uint32_t b = B0 + s_off[j];
                     len = s_off[j + 1] - s_off[j];
                     if (len <= (uint32_t)SMALL)
-                        sort_short_row(key2 + b, HAS_VAL ? val2 + b : nullptr, b, len, (uint64_t)(row0 + j), emit);
+                        sort_short_row<SMALL>(key2 + b, HAS_VAL ? val2 + b : nullptr, b, len, (uint64_t)(row0 + j), emit);
                 }
-                list_long_rows(valid, len, (uint32_t)(row0 + j), longs);
+                list_long_rows<SMALL>(valid, len, (uint32_t)(row0 + j), longs);
             }
         }
         __syncthreads();
@@ -543,8 +551,7 @@ constexpr int STAGE_ROW_AVG = 8;             // pass C staged while rows average
 // Pass C staged: a thread sorts rows of up to 8 entries in place; the entries of rows of 9 to 256
 // find their places by counting, as in fine_kernel.  (A warp per such row, and the bucket waiting
 // for its longest, took 1374 us for 2M rows of Poisson(7) lengths against 599, and 605 against 391 for
-// Poisson(5).  A 16-key in-place thread sort, which at this kernel's 64 registers ran mostly from
-// spilled registers, left rows of 9 to 16 entries unsorted and corrupted the index array on GB300.)
+// Poisson(5).)
 constexpr int STAGE_SMALL = 8;
 
 // The CTA copies the bytes [src, src + bytes) to dst, both 16-byte aligned, in 16-byte
@@ -740,7 +747,7 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
                     if (len <= (uint32_t)STAGE_SMALL) sort_idx_short(s_rec, s_idx + o, len);
                     else if (len <= (uint32_t)WARP_MAX) s_mid = 1;
                 }
-                list_long_rows(valid && len > (uint32_t)WARP_MAX, len, (uint32_t)(row0 + j), longs);
+                list_long_rows<WARP_MAX>(valid && len > (uint32_t)WARP_MAX, len, (uint32_t)(row0 + j), longs);
             }
             __syncthreads();
             const bool mid = s_mid != 0;  // uniform
@@ -779,9 +786,9 @@ fine_stage_kernel(int64_t major_n, Coarse co, int cap, const uint32_t *__restric
                     const uint32_t b2 = B0 + s_off[j];
                     len = s_off[j + 1] - s_off[j];
                     if (len <= (uint32_t)SMALL)
-                        sort_short_row(key2 + b2, HAS_VAL ? val2 + b2 : nullptr, b2, len, (uint64_t)(row0 + j), emit);
+                        sort_short_row<SMALL>(key2 + b2, HAS_VAL ? val2 + b2 : nullptr, b2, len, (uint64_t)(row0 + j), emit);
                 }
-                list_long_rows(valid, len, (uint32_t)(row0 + j), longs);
+                list_long_rows<SMALL>(valid, len, (uint32_t)(row0 + j), longs);
             }
         }
         __syncthreads();
@@ -823,15 +830,16 @@ __global__ void small_kernel(int64_t major_n, const uint32_t *__restrict__ start
             const uint32_t b = start[r];
             len = start[r + 1] - b;
             emit.pointer(r, b);
-            if (len <= (uint32_t)SMALL) sort_short_row<Emit, NoValue>(keys + b, nullptr, b, len, (uint64_t)r, emit);
+            if (len <= (uint32_t)SMALL_UNBOUNDED)
+                sort_short_row<SMALL_UNBOUNDED, Emit, NoValue>(keys + b, nullptr, b, len, (uint64_t)r, emit);
         }
-        list_long_rows(valid, len, (uint32_t)r, longs);
+        list_long_rows<SMALL_UNBOUNDED>(valid, len, (uint32_t)r, longs);
     }
 }
 
 // ---- long rows (both forms) --------------------------------------------------
 
-// Warp per listed row of (SMALL, WARP_MAX] entries: the row's keys in shared memory, each
+// Warp per listed row of up to WARP_MAX entries: the row's keys in shared memory, each
 // entry's rank = the number of smaller keys; values (when carried) move with their keys.
 template <class VT, class Emit>
 __global__ void __launch_bounds__(WARP_CTA_THREADS)
