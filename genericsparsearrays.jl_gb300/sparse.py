@@ -533,9 +533,9 @@ _SMALL_PTR = {key: buf.ctypes.data for key, buf in _SMALL.items()}
 
 def _mul_plain(C, A, B, alpha, beta) -> bool:
     """The usual call of mul_, or False with nothing done: a matrix (or its transpose / adjoint) whose
-    plan has been made, plain tensors on its device -- the current one -- of its element type, and
-    vectors or column-major matrices of sizes that agree.  Everything else, the errors among it, is
-    mul_'s.  It asks for the same things in fewer Python calls: a product of a small matrix waited 32
+    plan has been made, plain tensors on its device -- the current one -- of its element type, vectors
+    or matrices of sizes that agree, B in either order, C column-major.  Everything else, the errors
+    among it, is mul_'s.  It asks for the same things in fewer Python calls: a product of a small matrix waited 32
     us for its host code, most of it device and stream objects, ctypes wrappers and scalar arrays."""
     op, P = _lib.OP_N, A
     if isinstance(A, Transpose):
@@ -568,7 +568,7 @@ def _mul_plain(C, A, B, alpha, beta) -> bool:
     elif len(shape) == 2:
         r, k = shape
         opB, ldb = _layout(B)
-        if not ldb or opB != _lib.OP_N:
+        if not ldb:
             return False
     else:
         return False
@@ -598,7 +598,7 @@ def _mul_plain(C, A, B, alpha, beta) -> bool:
     lib = _lib.load()
     stream = _raw_stream(dev)
     head = (stream, code, icode, m, n, val.numel(), p0.data_ptr(), p1.data_ptr(), val.data_ptr(), BASE, op, k,
-            B.data_ptr(), ldb, _lib.OP_N, C.data_ptr(), ldc, al, be)
+            B.data_ptr(), ldb, opB, C.data_ptr(), ldc, al, be)
     if plan is not None:
         size = lib.gsa_plan_workspace_size(plan.handle, code, k)
         ws = torch.empty(size, dtype=torch.uint8, device=C.device) if size else None
