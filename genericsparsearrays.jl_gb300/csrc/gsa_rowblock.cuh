@@ -37,8 +37,9 @@ namespace gsa {
 // held to 32 registers (16 CTAs of 128 threads, every warp slot of the SM).  So are, less tightly,
 // the kernels of many columns of a column-major B, whose loads in flight otherwise take up to 128
 // registers (2048^2 grid; us unbounded / held): Float32 KC = 16 at 48 registers 250 / 161 (64: 167),
-// KC = 8 at 48 270 / 205, KC = 2 at 40 66 / 59 (32 registers spill: Poisson(10) rows 87 against 81),
-// ComplexF32 KC = 8 at 64 202 / 168.  Float64 KC = 8, taken for longer rows, is the faster unbounded
+// KC = 5 to 8 at 48 (KC = 8: 270 / 205), KC = 2 at 40 66 / 59 (32 registers spill: Poisson(10) rows 87
+// against 81), ComplexF32 KC = 5 to 8 at 64 (KC = 8: 202 / 168; KC = 6, which the compiler gave 45 and
+// loads one after another, on the 1024^2 grid 56 / 39).  Float64 KC = 8, taken for longer rows, is the faster unbounded
 // (Poisson(10) rows 383 against 453).  0 leaves the register count to the compiler.
 #ifndef GSA_RB_MIN_BLOCKS
 #define GSA_RB_MIN_BLOCKS 16
@@ -46,8 +47,8 @@ namespace gsa {
 template <typename V, int KC, int LAY> constexpr int rb_min_blocks() {
     if (KC * sizeof(V) <= 8 && (KC == 1 || LAY != COLUMNS)) return GSA_RB_MIN_BLOCKS;
     if (LAY != COLUMNS) return 0;
-    if (sizeof(V) == 4) return KC >= 8 ? 10 : (KC == 2 ? 12 : 0);
-    return std::is_same<V, cf32>::value && KC == 8 ? 8 : 0;
+    if (sizeof(V) == 4) return KC >= 5 ? 10 : (KC == 2 ? 12 : 0);
+    return std::is_same<V, cf32>::value && KC >= 5 ? 8 : 0;
 }
 // The bin order's ComplexF64 SpMV is held to 8 resident CTAs, which lets the compiler keep 64
 // registers (48 without the bound) and more loads in flight: power-law n = 10^6 160 us against
@@ -338,15 +339,21 @@ template <typename V, typename F> void by_layout(int KC, Layout lay, F &&f) {
         else f(kc, integral_constant<int, COLUMNS>{});
     };
     if constexpr (std::is_same<V, double>::value) {
-        if (lay == ANY) {  // odd numbers of columns (see launch_rowblock)
+        if (lay == ANY) {  // pairs (see launch_rowblock)
             f(integral_constant<int, 2>{}, integral_constant<int, ANY>{});
             return;
         }
     }
-    if constexpr (sizeof(V) == 4) {
-        if (KC == 16 && lay == COLUMNS) {
-            f(integral_constant<int, 16>{}, integral_constant<int, COLUMNS>{});
-            return;
+    if constexpr (!std::is_same<V, cf64>::value) {  // widths that are no power of two, and 16
+        if (lay == COLUMNS) {
+            using C = integral_constant<int, COLUMNS>;
+            if (KC == 3) { f(integral_constant<int, 3>{}, C{}); return; }
+            if (KC == 5) { f(integral_constant<int, 5>{}, C{}); return; }
+            if (KC == 6) { f(integral_constant<int, 6>{}, C{}); return; }
+            if (KC == 7) { f(integral_constant<int, 7>{}, C{}); return; }
+            if constexpr (sizeof(V) == 4) {
+                if (KC == 16) { f(integral_constant<int, 16>{}, C{}); return; }
+            }
         }
     }
     if (KC == 1) with(integral_constant<int, 1>{});
@@ -356,6 +363,7 @@ template <typename V, typename F> void by_layout(int KC, Layout lay, F &&f) {
 }
 
 // One launch over the k columns of B and C, KC per thread; k is a multiple of KC for lay = COLUMNS.
+// (launch_rowblock cuts a call into such launches.)
 template <typename V, typename I>
 int launch_columns(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t k, int KC, Layout lay, DenseIn<V> B,
                    const DenseOut<V> &C, const Plan *plan, void *ws, size_t ws_bytes) {
@@ -413,6 +421,24 @@ int launch_columns(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t k, int
     return check_cuda(cudaGetLastError(), "rowblock_kernel");
 }
 
+// The width of the next launch over a column-major B with `left` columns to go, W the best width of a
+// group: all of up to 8 columns; W where it divides them; else the largest width down to `least` (and no
+// less than half of W) that does, in one launch; else as many groups of W as there are.  Each launch
+// reads the matrix again and has its own start and last wave, which costs rows of 40 entries more than
+// it gives: halves of W for the rest (7 = 4 + 2 + 1) took, us against this rule, n = 6*10^4: Float32 7
+// columns 83 / 72, 15 columns 165 / 132, ComplexF32 5 columns 67 / 56, 12 columns 133 / 115; on the
+// 1024^2 grid Float32 3 columns 20 / 14, 7 columns 39 / 28, Float64 5 columns (pairs, one column
+// missing) 67 / 60.  Nine columns as 3 x 3 instead of 8 + 1, `least` = 3, give longer rows 3 to 19 %
+// (Float32 and ComplexF32; Float64 loses 12 % on Poisson(10) rows) and cost a grid 40 %.
+inline int next_width(int64_t left, int W, int least) {
+    if (W < 4) return left < W ? (int)left : W;  // a B too wide for L2: no more columns at a time
+    if (left <= 8) return (int)left;
+    if (left % W == 0) return W;
+    for (int w = W < 8 ? W : 8; w >= least; --w)
+        if (left % w == 0 && (w == 3 ? left == 9 : 2 * w >= (W < 8 ? W : 8))) return w;
+    return left >= W ? W : 8;
+}
+
 template <typename V, typename I>
 int launch_rowblock(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t k, DenseIn<V> B,
                     DenseOut<V> C, const Plan *plan, void *ws, size_t ws_bytes) {
@@ -436,38 +462,44 @@ int launch_rowblock(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t k, De
     // L2 (128 MB of it, 32 columns, n = 5*10^5, power law: 2451 us with 8 against 2192).  Row-major B (an entry's values share cache lines, and Float64 reads
     // them in 16-byte pieces): 8 columns (Float64 SpMM of the served mix's matrices, n = 10^6, k = 16:
     // 871 us with 8 against 982 us with 4); 4-byte values take 4.
-    const bool rowmajor = B.cs == 1 && B.rs > 1;
-    int KC = get_spmm_columns();
+    const bool rowmajor = B.cs == 1 && B.rs > 1, longer = a.nnz > G1_AVG * a.outer_n;
+    const int knob = get_spmm_columns();
+    int KC = knob;
     if (KC == 0) {
         if (rowmajor) KC = sizeof(V) >= 8 ? 8 : 4;
         else if (sizeof(V) == 4) KC = 16;
         else if (sizeof(V) == 16) KC = 1;
         else if (std::is_same<V, cf32>::value) KC = 8;
-        else if (a.nnz <= G1_AVG * a.outer_n) KC = 4;
+        else if (!longer) KC = 4;
         else KC = (size_t)a.inner_n * (size_t)k * sizeof(V) <= WIDE_B_BYTES ? 8 : 2;
     }
-    // A row-major B takes the smallest width that covers k, with columns missing in the last group.
-    // A column-major one takes the largest that k fills, and then the halves of it that the rest
-    // fills, a launch each: no kernel has to ask for missing columns.  A last single column of
-    // Float64 values would read the entries once more for one FMA each (power law, n = 5*10^5, 3
-    // columns 198 us against 161): odd k take pairs, the last one with a column missing.
+    // A row-major B takes the smallest width that covers k, with columns missing in the last group.  A
+    // column-major one takes widths that its columns fill (next_width), a launch for each: no kernel
+    // has to ask for missing columns.  Two exceptions, both Float64 by pairs in the general code: two
+    // columns of longer rows, whose fewer loads in flight are the faster (Poisson(10) rows, n = 3*10^5,
+    // 44 us against 48; power law, n = 2*10^5, 47 against 51; rows of 40 the same), and odd k where B is too
+    // wide for L2, whose last single column would read the entries once more for one FMA each.
     Layout lay = rowmajor ? ROWS : COLUMNS;
     if (rowmajor) {
         while (KC > 1 && KC / 2 >= k) KC >>= 1;
-    } else if (std::is_same<V, double>::value && k > 1 && (k & 1) && KC > 1) {
+    } else if (std::is_same<V, double>::value && !knob && k > 1 && ((k == 2 && longer) || (KC == 2 && (k & 1)))) {
         lay = ANY;
         KC = 2;
     }
+    const int least = longer && !std::is_same<V, double>::value ? 3 : 4;
     int rc = GSA_OK;
     timer_before(s);
     for (int64_t c = 0; c < k && !rc;) {
-        while (lay == COLUMNS && KC > k - c) KC >>= 1;
-        const int64_t cols = lay == COLUMNS ? (k - c) / KC * KC : k;
+        const int64_t left = k - c;
+        int w = KC;
+        if (lay == COLUMNS && !knob && !std::is_same<V, cf64>::value) w = next_width(left, KC, least);
+        while (lay == COLUMNS && w > left) w >>= 1;  // an explicit width, and ComplexF64: halves of it
+        const int64_t cols = lay == COLUMNS ? left / w * w : k;
         DenseIn<V> Bc = B;
         DenseOut<V> Cc = C;
         Bc.p += c * B.cs;
         Cc.p += c * C.ld;
-        rc = launch_columns<V, I>(s, a, cols, KC, lay, Bc, Cc, plan, ws, ws_bytes);
+        rc = launch_columns<V, I>(s, a, cols, w, lay, Bc, Cc, plan, ws, ws_bytes);
         c += cols;
     }
     timer_after(s);
