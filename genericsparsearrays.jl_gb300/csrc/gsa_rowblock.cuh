@@ -39,13 +39,16 @@ namespace gsa {
 // registers (2048^2 grid; us unbounded / held): Float32 KC = 16 at 48 registers 250 / 161 (64: 167),
 // KC = 5 to 8 at 48 (KC = 8: 270 / 205), KC = 2 at 40 66 / 59 (32 registers spill: Poisson(10) rows 87
 // against 81), ComplexF32 KC = 5 to 8 at 64 (KC = 8: 202 / 168; KC = 6, which the compiler gave 45 and
-// loads one after another, on the 1024^2 grid 56 / 39).  Float64 KC = 8, taken for longer rows, is the faster unbounded
+// loads one after another, on the 1024^2 grid 56 / 39).  Two 4-byte columns of a row-major B take 48
+// (32, which the two-stride code fitted, spill 184 bytes: power law, n = 2*10^5, 36 us against 34; rows of 40
+// 26 against 22).  Float64 KC = 8, taken for longer rows, is the faster unbounded
 // (Poisson(10) rows 383 against 453).  0 leaves the register count to the compiler.
 #ifndef GSA_RB_MIN_BLOCKS
 #define GSA_RB_MIN_BLOCKS 16
 #endif
 template <typename V, int KC, int LAY> constexpr int rb_min_blocks() {
-    if (KC * sizeof(V) <= 8 && (KC == 1 || LAY != COLUMNS)) return GSA_RB_MIN_BLOCKS;
+    if (KC == 1 && sizeof(V) <= 8) return GSA_RB_MIN_BLOCKS;
+    if (LAY == ROWS && KC == 2 && sizeof(V) == 4) return 10;
     if (LAY != COLUMNS) return 0;
     if (sizeof(V) == 4) return KC >= 5 ? 10 : (KC == 2 ? 12 : 0);
     return std::is_same<V, cf32>::value && KC >= 5 ? 8 : 0;
@@ -327,13 +330,23 @@ binned_kernel(CompressedArgs<V, I> a, int64_t k, DenseIn<V> B, DenseOut<V> C, in
 
 constexpr size_t WIDE_B_BYTES = (size_t)96 << 20;  // of the 129 MB L2: a B that stays there beside the entries
 
-// Calls f(columns per thread, layout of B), both as compile-time constants.  The FP64 types keep
+// Calls f(columns per thread, layout of B), both as compile-time constants.  The FP64 types alone keep
 // the general code for a row-major B (its columns are one cache line, so waiting for them in turn
 // costs little, and the registers of the other form do: ComplexF64 grid, 16 columns 694 us against
 // 731, Float64 200 against 231).
 template <typename V, typename F> void by_layout(int KC, Layout lay, F &&f) {
-    constexpr Layout R = sizeof(V) == 4 || std::is_same<V, cf32>::value ? ROWS : ANY;
     using std::integral_constant;
+    constexpr Layout R = std::is_same<V, double>::value || std::is_same<V, cf64>::value ? ANY : ROWS;
+    if constexpr (std::is_same<V, int64_t>::value) {
+        if (lay == ANY) {  // a row-major B, short rows (see launch_rowblock)
+            using A = integral_constant<int, ANY>;
+            if (KC == 1) f(integral_constant<int, 1>{}, A{});
+            else if (KC == 2) f(integral_constant<int, 2>{}, A{});
+            else if (KC == 4) f(integral_constant<int, 4>{}, A{});
+            else f(integral_constant<int, 8>{}, A{});
+            return;
+        }
+    }
     auto with = [&](auto kc) {
         if (lay == ROWS) f(kc, integral_constant<int, R>{});
         else f(kc, integral_constant<int, COLUMNS>{});
@@ -459,14 +472,25 @@ int launch_rowblock(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t k, De
     // bound by the FP64 pipe, 1343 / 1377 / 1372 / 1372 and 858 / 885 / 919 / 973.  Hence 16 for 4-byte
     // values, 8 for ComplexF32 and for Float64 (and Int64) rows of several lanes, 4 for shorter
     // ones, 1 for ComplexF64; and 2 for the Float64 rows of several lanes where B does not stay in
-    // L2 (128 MB of it, 32 columns, n = 5*10^5, power law: 2451 us with 8 against 2192).  Row-major B (an entry's values share cache lines, and Float64 reads
-    // them in 16-byte pieces): 8 columns (Float64 SpMM of the served mix's matrices, n = 10^6, k = 16:
-    // 871 us with 8 against 982 us with 4); 4-byte values take 4.
+    // L2 (128 MB of it, 32 columns, n = 5*10^5, power law: 2451 us with 8 against 2192).
+    // Row-major B (an entry's values share cache lines, and Float64 reads them in 16-byte pieces): 8
+    // columns for the FP64 types (Float64 SpMM of the served mix's matrices, n = 10^6, k = 16: 871 us with
+    // 8 against 982 us with 4).  The others, KC = 4 / 8, us on the 1024^2 grid, Poisson(10) rows (n =
+    // 3*10^5), the power law (2*10^5) and Poisson(40) rows (6*10^4): Float32, 8 columns 62 / 56, 60 / 62, 73 / 75,
+    // 49 / 51, 12 columns 77 / 83, 75 / 83, 91 / 109, 69 / 78; ComplexF32, 5 columns 54 / 46, 53 / 48, 71 / 76, 52 /
+    // 44, 8 columns 95 / 93, 82 / 85, 96 / 102, 68 / 75, 16 columns 297 / 293, 196 / 202, 212 / 213, 163 / 177, 31 columns
+    // 315 / 270, 260 / 243, 313 / 310, 190 / 187; Int64's longer rows 5 columns 56 / 52, 86 / 77, 53 / 44, 12 columns
+    // 107 / 117, 131 / 158, 94 / 106, 31 columns 291 / 262, 362 / 354, 193 / 190.  Hence 4 for 4-byte values, but
+    // 8 where that makes one group of a grid's; and 8 for 8-byte values, but 4 for 8 to 23 columns of
+    // longer rows.
     const bool rowmajor = B.cs == 1 && B.rs > 1, longer = a.nnz > G1_AVG * a.outer_n;
     const int knob = get_spmm_columns();
     int KC = knob;
     if (KC == 0) {
-        if (rowmajor) KC = sizeof(V) >= 8 ? 8 : 4;
+        if (rowmajor && sizeof(V) == 4) KC = !longer && k > 4 && k <= 8 ? 8 : 4;
+        else if (rowmajor && (std::is_same<V, cf32>::value || std::is_same<V, int64_t>::value))
+            KC = longer && k >= 8 && k < 24 ? 4 : 8;
+        else if (rowmajor) KC = 8;
         else if (sizeof(V) == 4) KC = 16;
         else if (sizeof(V) == 16) KC = 1;
         else if (std::is_same<V, cf32>::value) KC = 8;
@@ -479,8 +503,11 @@ int launch_rowblock(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t k, De
     // columns of longer rows, whose fewer loads in flight are the faster (Poisson(10) rows, n = 3*10^5,
     // 44 us against 48; power law, n = 2*10^5, 47 against 51; rows of 40 the same), and odd k where B is too
     // wide for L2, whose last single column would read the entries once more for one FMA each.
+    // (Int64 and a row-major B: the loads of a row's columns issued together pay on longer rows -- power
+    // law, 7 columns 179 us / 86 -- but not on a grid's, 2 columns 21.6 us / 23.6, 12 columns 111 / 116.)
     Layout lay = rowmajor ? ROWS : COLUMNS;
     if (rowmajor) {
+        if (std::is_same<V, int64_t>::value && !longer) lay = ANY;
         while (KC > 1 && KC / 2 >= k) KC >>= 1;
     } else if (std::is_same<V, double>::value && !knob && k > 1 && ((k == 2 && longer) || (KC == 2 && (k & 1)))) {
         lay = ANY;
