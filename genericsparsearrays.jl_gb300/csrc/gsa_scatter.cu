@@ -302,10 +302,19 @@ int launch_scatter_block(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t 
     // bound the kernel.  Measured with KC = 2 / 4, us (adjoints, Int32 indices): Poisson(10) rows, n =
     // 10^5, 5 and 8 columns ComplexF32 37.5 / 42.0 and 52.6 / 60.7, Float64 37.8 / 47.2 and 52.2 / 56.2,
     // Float32 36.7 / 43.0 and 48.3 / 50.2; 1024^2 grid, 8 columns ComplexF32 91 / 93, Float64 117.5 /
-    // 117.5, Float32 56 / 48; three columns 30.4 / 25.8, 30.6 / 27.5 and 28.7 / 25.5 on the Poisson rows.
-    // Hence 2 for values of 8 bytes and more, 4 for three columns and for 4-byte values.
+    // 117.5, Float32 56 / 48; three columns, one group with one column idle against two, 30.4 / 25.8,
+    // 30.6 / 27.5 and 28.7 / 25.5 on the Poisson rows (seven, with as many idle in either: ComplexF32 78 / 78 on
+    // the grid, 108 / 108 and 99 / 103 on Poisson(10) and Poisson(40) rows).  Int64, whose adds are the cheaper:
+    // 1024^2 grid, 4, 7, 8 and 9 columns 44 / 40, 81 / 70, 88 / 77 and 102 / 91; Poisson(40) rows, 5 to 9 columns
+    // 75 / 92, 83 / 97, 95 / 102, 121 / 107 and 131 / 127.
+    // Hence 4 for 4-byte values and for three columns; 2 for other values of 8 bytes and more, but for
+    // Int64 only where four would leave most of a second group idle (5 to 7 columns) of longer rows.
     int KC = get_spmm_columns();
-    if (KC == 0) KC = sizeof(V) >= 16 ? 2 : (sizeof(V) == 8 && k != 3 ? 2 : 4);
+    if (KC == 0) {
+        const bool int64 = std::is_same<V, int64_t>::value;
+        const bool two = !int64 || (k > 4 && k < 8 && a.nnz > G1_AVG * a.outer_n);
+        KC = sizeof(V) >= 16 ? 2 : (sizeof(V) == 8 && k != 3 && two ? 2 : 4);
+    }
     if (k == 1) KC = 1;
     if (KC > k) KC = k <= 2 ? 2 : (k <= 4 ? 4 : 8);
     const int64_t ncg = ceil_div(k, KC);
