@@ -74,6 +74,7 @@ SIGNATURES = {
     "gsa_csr_spmv_noalloc": ([_vp, _i32, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _i32, _vp, _vp,
                               _vp, _vp], _i32),
     "gsa_mul_workspace_size": ([_i32, _i32, _i32, _i64, _i64, _i64, _i32, _i64, _i32], _sz),
+    "gsa_grouped_columns": ([_i32, _vp, _i64], _i32),
     "gsa_grouped_tiles": ([_i32, _vp, _i64, _i32, ctypes.POINTER(_i64)], _i32),
     "gsa_grouped_mul": ([_vp, _i32, _i32, _i32, _vp, _i64, _i64, _i32, _i32], _i32),
     "gsa_batch_create": ([_vp, _i32, _i32, _i32, _vp, _i64, _i32, _i32, ctypes.POINTER(_vp)], _i32),

@@ -186,6 +186,8 @@ class GroupedLauncher:
             slot.update(self._alloc(max(len(products), 2 * slot["cap"])))
         view = slot["host"].numpy().view(ITEM_DTYPE)
         items, dt, it = pack_items(products, out=view)
+        if not columns:
+            columns = _lib.load().gsa_grouped_columns(_DTYPE[dt], items.ctypes.data_as(ctypes.c_void_p), items.size)
         ntiles = tiles(items, dt, columns)
         nbytes = len(products) * ITEM_DTYPE.itemsize
         with torch.cuda.stream(stream), torch.cuda.device(self.device):

@@ -20,10 +20,26 @@ namespace gsa {
 
 static_assert(sizeof(gsa_group_item) == 144, "gsa_group_item layout");
 
-// Columns per thread where the caller leaves them open (column-major B).  ComplexF64, bound by the
-// FP64 pipe, takes one: with four, a warp's items of one column ran the four-column code
-// (4096 banded products of 1, 4 or 8 columns: 5.4 ms against 4.4).
+// Columns per thread where the caller leaves them open and nothing is known of the items.
 int default_columns(int dtype) { return dtype_size(dtype) == 16 ? 1 : (dtype_size(dtype) == 8 ? 2 : 4); }
+
+// Columns per thread for these items.  ComplexF64 is bound by the FP64 pipe, and a column missing in a
+// group costs it as much as one that is there, so the choice is between one and two.  256 products, us with
+// 1 / 2 / 4: column-major B, 1 column 68 / 68 / 75, 2 104 / 109 / 110, 3 141 / 177 / 148, 4 193 / 180 / 189, 8
+// 353 / 325 / 345, 16 645 / 594 / 605, a mix of 1, 4 and 8 188 / 192 / 235; row-major B 66 / 68 / 75, 106 / 103 /
+// 105, 145 / 178 / 148, 198 / 177 / 183, 374 / 328 / 327, 686 / 601 / 598, 199 / 194 / 223.  Hence the cheaper by
+// those rates: a column alone costs 1.08 (column-major) or 1.13 of one in a pair from four columns on.
+int columns_for(int dtype, const gsa_group_item *items, int64_t count) {
+    if (dtype_size(dtype) != 16) return default_columns(dtype);
+    double one = 0, two = 0;
+    for (int64_t i = 0; i < count; ++i) {
+        const double entries = (double)items[i].nnz, k = (double)items[i].k;
+        const bool many = items[i].k >= 4;
+        one += entries * k * (many ? (items[i].b_rowmajor ? 1.13 : 1.08) : 1.0);
+        two += entries * 2 * ceil(k / 2) * (many ? 1.0 : 1.04);
+    }
+    return two < one ? 2 : 1;
+}
 
 struct GroupedBody {
     cudaStream_t s; const gsa_group_item *items; int64_t count, ntiles; int base, KC, g1;
@@ -60,6 +76,10 @@ struct gsa_batch {
 };
 
 extern "C" {
+
+int gsa_grouped_columns(int dtype, const gsa_group_item *items, int64_t count) {
+    return columns_for(dtype, items, items && count > 0 ? count : 0);
+}
 
 int gsa_grouped_tiles(int dtype, gsa_group_item *items, int64_t count, int columns, int64_t *ntiles) {
     if (!dtype_size(dtype)) return fail(GSA_ERR_UNSUPPORTED, "unsupported dtype %d", dtype);
@@ -122,7 +142,7 @@ int gsa_batch_create(void *stream, int dtype, int itype, int base, const gsa_gro
     b->dtype = dtype;
     b->itype = itype;
     b->base = base;
-    b->columns = columns;
+    b->columns = columns == 0 ? columns_for(dtype, items, count) : columns;
     b->g1 = g1_avg;
     b->host.assign(items, items + count);
     for (int64_t i = 0; itype == GSA_IDX32 && i < count; ++i)
@@ -131,7 +151,7 @@ int gsa_batch_create(void *stream, int dtype, int itype, int base, const gsa_gro
             return fail(GSA_ERR_INVALID_ARG, "item %lld: nnz exceeds what Int32 indices can address",
                         (long long)i);
         }
-    int rc = gsa_grouped_tiles(dtype, b->host.data(), count, columns, &b->ntiles);
+    int rc = gsa_grouped_tiles(dtype, b->host.data(), count, b->columns, &b->ntiles);
     if (!rc && count > 0x7fffffffLL) rc = fail(GSA_ERR_UNSUPPORTED, "batch: more than 2^31 - 1 items");
     std::vector<int32_t> table;
     if (!rc && count > 0) {

@@ -404,8 +404,12 @@ typedef struct {
  * bin order, or has rows of more than 512 entries). */
 int gsa_plan_bin_order(const gsa_plan *plan, const void **view, int64_t *warps);
 
+/* Columns per thread that suit these items (host memory): by dtype, and for ComplexF64 by their
+ * columns, entries and layouts of B. */
+int gsa_grouped_columns(int dtype, const gsa_group_item *items, int64_t count);
+
 /* Checks the items (host memory), fills first_tile and returns the tile count.
- * columns: right-hand-side columns a thread accumulates (0 = by dtype, 1, 2, 4, 8);
+ * columns: right-hand-side columns a thread accumulates (0 = by dtype alone, 1, 2, 4, 8);
  * the launch must use the same value. */
 int gsa_grouped_tiles(int dtype, gsa_group_item *items, int64_t count, int columns, int64_t *ntiles);
 
@@ -416,7 +420,8 @@ int gsa_grouped_mul(void *stream, int dtype, int itype, int base, const gsa_grou
                     int64_t count, int64_t ntiles, int columns, int g1_avg);
 
 /* A batch: the items copied to the device once (one allocation, synchronizes the
- * stream), run many times with new contents of the same B and C buffers. */
+ * stream), run many times with new contents of the same B and C buffers.  columns = 0 is
+ * gsa_grouped_columns of its items. */
 typedef struct gsa_batch gsa_batch;
 typedef enum {
     GSA_BATCH_GROUPED = 0,   /* one grouped launch */
