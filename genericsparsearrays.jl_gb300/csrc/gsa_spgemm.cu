@@ -122,7 +122,9 @@ __device__ __forceinline__ uint64_t open_rows(const I *__restrict__ pi, const I 
 // increasing order after take(c, at) for each of its products in the reference's order (entries in
 // order, each Q row in order).  False, with part of them visited, when a Q row is not sorted, or has
 // the column that the end mark stands for.  Bound by its instructions: K is 5 for the warps whose
-// rows have no more entries (a grid's): 212 us against 250 with 8 for count_rows_kernel on the 2048^2 grid.
+// rows have no more entries: 212 us against 250 with 8 for count_rows_kernel on the 2048^2 grid, its whole
+// product 780 against 847; on Poisson(2) to Poisson(10) rows, where few warps have such rows alone, the
+// two are within 1 %.
 // (A second column held per cursor, loaded one advance ahead, was slower: 591 us against 510 for
 // merge_rows_kernel, for its registers.)
 template <typename I, int K, typename Take, typename Visit>
@@ -376,22 +378,22 @@ tiny_kernel(const uint32_t *__restrict__ list, const uint32_t *__restrict__ coun
             }
             P = P + len < (uint32_t)SG_TINY_P ? P + len : (uint32_t)SG_TINY_P;
         };
-        if (e - b <= SG_TINY_A) {
-            // rows of up to SG_TINY_A entries: their indices, Q-row bounds and values loaded
-            // together first, so the loads overlap instead of forming one chain per entry
+        for (int64_t t0 = b; t0 < e; t0 += SG_TINY_A) {
+            // SG_TINY_A entries at a time: their indices, Q-row bounds and values loaded together
+            // first, so the loads overlap instead of forming one chain per entry
             int64_t qb[SG_TINY_A];
             uint32_t len[SG_TINY_A];
             V a[SG_TINY_A];
 #pragma unroll
             for (int c = 0; c < SG_TINY_A; ++c) {
-                const int64_t t = b + c;
+                const int64_t t = t0 + c;
                 qb[c] = (int64_t)(t < e ? __ldg(pi + t) : (I)0) - base;  // k for now
                 if constexpr (NUMERIC) a[c] = t < e ? ldg(pv + t) : V{};
             }
 #pragma unroll
             for (int c = 0; c < SG_TINY_A; ++c) {
                 const int64_t k = qb[c];
-                const bool ok = b + c < e && (uint64_t)k < (uint64_t)q_outer;
+                const bool ok = t0 + c < e && (uint64_t)k < (uint64_t)q_outer;
                 const int64_t q0 = ok ? (int64_t)__ldg(qp + k) - base : 0;
                 len[c] = ok ? (uint32_t)((int64_t)__ldg(qp + k + 1) - base - q0) : 0u;
                 qb[c] = q0;
@@ -399,16 +401,6 @@ tiny_kernel(const uint32_t *__restrict__ list, const uint32_t *__restrict__ coun
 #pragma unroll
             for (int c = 0; c < SG_TINY_A; ++c)
                 if (len[c]) expand(qb[c], len[c], NUMERIC ? a[c] : V{});
-        } else {
-            for (int64_t t = b; t < e; ++t) {
-                const int64_t k = (int64_t)__ldg(pi + t) - base;
-                if ((uint64_t)k >= (uint64_t)q_outer) continue;
-                const int64_t q0 = (int64_t)__ldg(qp + k) - base;
-                const uint32_t l = (uint32_t)((int64_t)__ldg(qp + k + 1) - base - q0);
-                V av{};
-                if constexpr (NUMERIC) av = ldg(pv + t);
-                expand(q0, l, av);
-            }
         }
         uint32_t firsts = 0;
         for (uint32_t s2 = 0; s2 < P; ++s2) {
