@@ -472,7 +472,9 @@ int launch_rowblock(cudaStream_t s, const CompressedArgs<V, I> &a, int64_t k, De
     // bound by the FP64 pipe, 1343 / 1377 / 1372 / 1372 and 858 / 885 / 919 / 973.  Hence 16 for 4-byte
     // values, 8 for ComplexF32 and for Float64 (and Int64) rows of several lanes, 4 for shorter
     // ones, 1 for ComplexF64; and 2 for the Float64 rows of several lanes where B does not stay in
-    // L2 (128 MB of it, 32 columns, n = 5*10^5, power law: 2451 us with 8 against 2192).
+    // L2: KC = 2 / 4 / 8, n = 5*10^5, Poisson(10) rows with 76 MB of B 685 / 605 / 609, 91 MB 935 / 877 / 911, 106 MB
+    // 1240 / 1188 / 1282, 122 MB 1570 / 1555 / 1635, 183 MB 3176 / 3192 / 3264; the power law 938 / 860 / 861, 1273 /
+    // 1249 / 1339, 1698 / 1692 / 1891, 2187 / 2223 / 2424, 4706 / 4668 / 4825 (Int64: all alike from 91 MB on).
     // Row-major B (an entry's values share cache lines, and Float64 reads them in 16-byte pieces): 8
     // columns for the FP64 types (Float64 SpMM of the served mix's matrices, n = 10^6, k = 16: 871 us with
     // 8 against 982 us with 4).  The others, KC = 4 / 8, us on the 1024^2 grid, Poisson(10) rows (n =

@@ -18,8 +18,9 @@
 // * rmul_or_fill: LinearAlgebra._rmul_or_fill!(C, beta) as the reference calls
 //   it before its atomic kernels (src/matrix_csr/matrix_csr.jl:192).
 //
-// Complex values use one atomic per component (the reference's KA @atomic
-// cannot do Complex, so its CSR-T / CSC-N / COO products skip Complex).
+// ComplexF32 values are added by one vector reduction, ComplexF64 by one atomic per
+// component (the reference's KA @atomic cannot do Complex, so its CSR-T / CSC-N / COO
+// products skip Complex).
 #include "gsa_rows.cuh"
 
 namespace gsa {
